@@ -6,7 +6,8 @@
 //
 // C(i,j) -= sum_k A(i,k) B(k,j) with A(i,k) = U[k, i] and B(k,j) = W[k, j].
 // Arithmetics:
-//   FP64          FP64 tensor cores: mma.sync.m16n8k8.f64 from shared-memory
+//   FP64          integer tensor cores on 8-bit digits for large panels
+//                 (update_i8.cu), else FP64 tensor cores: mma.sync.m16n8k8.f64 from shared-memory
 //                 tiles staged with cp.async (double-buffered); 64x64 C tile
 //                 per CTA, 32x32 per warp.
 //   FP64_ORDERED  SIMT, every product and sum rounded separately with k
@@ -29,6 +30,7 @@
 #include <type_traits>
 
 #include "bbk_internal.cuh"
+#include "umma.cuh"
 
 namespace bbk {
 namespace {
@@ -57,6 +59,8 @@ struct UpdArgs {
   // BF16 mode: per 64-block power-of-two scales of A rows and B columns
   const double* a_scale;
   const double* b_scale;
+  // panel mode: run only when this flag is set (null: always)
+  const int* gate;
 };
 
 __device__ __forceinline__ void cp_async_8(double* smem_dst, const double* gsrc, bool valid) {
@@ -82,6 +86,7 @@ __device__ __forceinline__ void cp_async_wait() {
 __device__ __forceinline__ bool resolve_range(UpdArgs& U) {
   if (U.st == nullptr) return true;
   if (ld_relaxed_s32(&U.st->abort)) return false;
+  if (U.gate != nullptr && ldcg(U.gate) == 0) return false;
   const int k0 = ldcg(&U.st->kstart[U.panel & 1]);
   const int e = ldcg(&U.st->kstart[(U.panel + 1) & 1]);
   U.inner = e - k0;
@@ -527,6 +532,7 @@ __global__ void __launch_bounds__(Wide<BM, BN, WM, WN, Stages, BK, MinBlocks>::k
     // panel mode: range from the device state, tiles from the BN-aligned
     // row at or below the trailing matrix's first row
     if (ld_relaxed_s32(&U.st->abort)) return;
+    if (U.gate != nullptr && ldcg(U.gate) == 0) return;
     const int k0 = ldcg(&U.st->kstart[U.panel & 1]);
     const int e = ldcg(&U.st->kstart[(U.panel + 1) & 1]);
     U.inner = e - k0;
@@ -1157,19 +1163,6 @@ struct USmem {
 };
 static_assert(2 * USmem<3>::kBytes + 2048 <= 228 * 1024, "two CTAs per SM");
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Shared-memory matrix descriptor, SWIZZLE_NONE K-major: start address,
-// leading (k-direction, 128 B) and stride (row-direction) byte offsets,
-// version 1.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t sbo) {
-  constexpr uint64_t kLbo = 128 >> 4;
-  return (static_cast<uint64_t>((saddr >> 4) & 0x3FFF)) | (kLbo << 16) |
-         (static_cast<uint64_t>(sbo >> 4) << 32) | (1ull << 46);
-}
-
 // Instruction descriptor of kind::f16: FP32 accumulate, BF16 A and B, both
 // K-major, N = 128, M = 128.
 constexpr uint32_t kUIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kUN >> 3) << 17) |
@@ -1180,35 +1173,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
       "l"(da), "l"(db), "r"(kUIdesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(done)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Bounded wait for phase `parity` of mbarrier `mbar`: false when it ran out
-// (or another kernel of the factorization aborted).
-__device__ bool mbar_wait(uint32_t mbar, uint32_t parity, const DeviceState* st, unsigned long long timeout_ns) {
-  unsigned long long t0 = 0;
-  for (unsigned it = 1;; ++it) {
-    if (mbar_try(mbar, parity)) return true;
-    if ((it & 63u) == 0) {
-      const unsigned long long now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > timeout_ns || ld_relaxed_s32(&st->abort)) return false;
-    }
-  }
 }
 
 // Roles (warp-specialized, no CTA barrier inside the main loop):
@@ -1227,10 +1191,6 @@ __device__ bool mbar_wait(uint32_t mbar, uint32_t parity, const DeviceState* st,
 constexpr int kUEpi = 4, kUProd = 1;
 constexpr int kUWarps = kUEpi + kUProd + 1;
 constexpr int kUBlock = kUWarps * 32;
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
 
 template <int kTerms>
 __global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U, const __nv_bfloat16* ah,
@@ -1689,6 +1649,13 @@ int launch_update(const FactorPlan& plan, int panel, cudaStream_t s) {
     return plan.mode == BBK_UPDATE_BF16
                ? launch_bf16_split<1>(U, buf, plan.kpad, plan.hstride, grid_mma, vec, plan.n - nominal_e, s)
                : launch_bf16_split<3>(U, buf, plan.kpad, plan.hstride, grid_mma, vec, plan.n - nominal_e, s);
+  }
+  // large updates on the integer tensor cores; an explicit tile shape keeps
+  // the FP64 ones
+  static const bool digits = getenv("BBK_UPDATE_TILE") == nullptr;
+  if (plan.mode == BBK_UPDATE_FP64 && vec && digits) {
+    const int rc = launch_update_i8(plan, panel, plan.n - nominal_e, &U.gate, s);
+    if (rc) return rc;
   }
   if (plan.mode == BBK_UPDATE_FP64 && vec) {
     bool launched = false;
