@@ -37,10 +37,22 @@
 // row as keeping its pivot would leave it and reduces that row's argmax in
 // the same exchange, so when the pivot is kept (most steps of saddle-point
 // matrices) the next step starts without a row exchange.
+//
+// A step is bound by the length of its instruction stream and the exchanges,
+// not by arithmetic or memory: one or two warps per scheduler, about 1 100
+// instructions each.  So quotients that every thread used to form go to the
+// communication warp, one per lane; the owner of a slot is a multiplication;
+// and the sums over the rows run for exactly the slots' 32-wide chunks.
+// Panels of up to a few thousand columns run on one thread-block cluster.
+// KKT n = 10000, block 128: 50.1 -> 42.5 ms per factorization (4.2 us per
+// pivot); KKT n = 1999, block 64: 9.3 -> 6.3 ms; n = 40000, block 256: 384 ->
+// 362 ms.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
+#include <type_traits>
 
 #include "bbk_internal.cuh"
 
@@ -58,6 +70,9 @@ constexpr int kBlock = kThreads + 32;   // compute warps + the communication war
 constexpr int kCols = 3;  // slots per thread: S <= kCols * kThreads
 constexpr int kPairSlots = 96;  // slots per CTA up to which the warps split the candidate sums by rows
 constexpr int kAllWarps = kBlock / 32;
+constexpr int kClusterMax = 16;      // CTAs of a cluster panel
+constexpr int kClusterSlots = 224;   // slots per CTA of a cluster panel: 7 per lane
+constexpr int kClusterWords = 5 + kMaxPub;  // record: two argmaxes and the published doubles
 constexpr int kMaxGrid = kBlock;  // CTAs of a panel launch: every thread reads one record
 constexpr int kRecA = 4;  // argmax words of a record: idx, value hi, value lo, slot
 constexpr int kRecB = 6;  // second argmax: idx, value hi, value lo, slot, payload hi, payload lo
@@ -159,6 +174,25 @@ __device__ __forceinline__ void warp_argmax(Cand& c) {
   if (kPay) c.pay = __shfl_sync(0xffffffffu, c.pay, who);
 }
 
+// Warp-wide maximum of values that are never negative or NaN.
+__device__ __forceinline__ double warp_max(double v) {
+  const unsigned long long key = static_cast<unsigned long long>(__double_as_longlong(v));
+  const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+  return __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(mhi) << 32) | mlo));
+}
+
+// The first channel of an exchange: an argmax, or with kTwo only a maximum
+// (the candidate column's).
+template <bool kTwo>
+__device__ __forceinline__ void warp_channel_a(Cand& c) {
+  if (kTwo)
+    c.v = warp_max(c.v);
+  else
+    warp_argmax<false>(c);
+}
+
 // Shared memory of the exchanges.
 struct XShared {
   Cand pa[kWarps], pb[kWarps];        // this CTA's record: the compute warps' partials
@@ -188,7 +222,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // `cb` with kTwo) over the CTA, publish the CTA's record (the reductions plus
 // the npub doubles of pub_in), and return the grid-wide argmax of every
 // channel once all `nslots` CTAs of this exchange have arrived; X.pub[k] then
-// holds pub_in[k] of CTA pub_owner[k].  Must be called by every thread.
+// holds pub_in[k] of CTA pub_owner(k).  Must be called by every thread.
 //
 // Records are structure-of-arrays: word w of CTA c lives at
 // slots[((tag & 1) * kSlotWords + w) * slot_stride + c], so one warp load
@@ -206,14 +240,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // release fence (here when `release`, or earlier by the caller, after a CTA
 // barrier that follows the writes to publish), so after the exchange this
 // CTA sees everything the other CTAs wrote before their fence.
-template <bool kTwo>
+template <bool kTwo, typename OwnerOf>
 __device__ __forceinline__ XResult exchange(const PanelArgs& P, unsigned tag, bool release, Cand ca, Cand cb,
-                                            const double* pub_in, const int (&pub_owner)[kMaxPub], int npub,
-                                            XShared& X) {
+                                            const double* pub_in, OwnerOf&& pub_owner, int npub, XShared& X) {
   constexpr int kRec = kRecA + (kTwo ? kRecB : 0);
   const int t = threadIdx.x;
   const int lane = t & 31, warp = t >> 5;
-  warp_argmax<false>(ca);
+  warp_channel_a<kTwo>(ca);
   if (kTwo) warp_argmax<true>(cb);
   if (lane == 0 && warp < kWarps) {
     X.pa[warp] = ca;
@@ -229,7 +262,7 @@ __device__ __forceinline__ XResult exchange(const PanelArgs& P, unsigned tag, bo
     // one compute warp's partial per lane, reduced across the warp
     Cand a = lane < kWarps ? X.pa[lane] : no_cand();
     Cand b = kTwo && lane < kWarps ? X.pb[lane] : no_cand();
-    warp_argmax<false>(a);
+    warp_channel_a<kTwo>(a);
     if (kTwo) warp_argmax<true>(b);
     if (lane == 0 && release) fence_acq_rel_gpu();
     if (lane < kRec + 2 * npub) {
@@ -282,10 +315,7 @@ __device__ __forceinline__ XResult exchange(const PanelArgs& P, unsigned tag, bo
   // yet this exchange's is read again (its store may land after the arrival).
   const bool has_rec = t < P.nslots;
   const bool has_pub = warp == kCommWarp && lane < npub;
-  int owner = 0;
-#pragma unroll
-  for (int k = 0; k < kMaxPub; ++k)
-    if (lane == k) owner = pub_owner[k];
+  const int owner = has_pub ? pub_owner(lane) : 0;
   const unsigned long long* rsrc = par_base + (has_rec ? t : 0);
   const unsigned long long* psrc =
       par_base + static_cast<size_t>(kRec + 2 * (has_pub ? lane : 0)) * st + (has_pub ? owner : 0);
@@ -327,7 +357,7 @@ __device__ __forceinline__ XResult exchange(const PanelArgs& P, unsigned tag, bo
       rb = Cand{join_hi_lo(w[5], w[6]), static_cast<int>(w[4] & 0xffffffffu),
                 static_cast<int>(w[7] & 0xffffffffu), join_hi_lo(w[8], w[9])};
   }
-  warp_argmax<false>(ra);
+  warp_channel_a<kTwo>(ra);
   if (kTwo) warp_argmax<true>(rb);
   const int wok = __all_sync(0xffffffffu, ok);
   if (lane == 0) {
@@ -340,21 +370,236 @@ __device__ __forceinline__ XResult exchange(const PanelArgs& P, unsigned tag, bo
   // every warp reduces the per-warp partials (one per lane)
   r.a = lane < kAllWarps ? X.ra[lane] : no_cand();
   r.b = kTwo && lane < kAllWarps ? X.rb[lane] : no_cand();
-  warp_argmax<false>(r.a);
+  warp_channel_a<kTwo>(r.a);
   if (kTwo) warp_argmax<true>(r.b);
   r.ok = __all_sync(0xffffffffu, lane >= kAllWarps || X.ok[lane] != 0);
   return r;
+}
+
+// The exchange of a panel that runs on one thread-block cluster: each CTA
+// stores its record straight into every CTA's shared memory, and the stores
+// complete that CTA's barrier; no global memory is involved.  Records and
+// barriers alternate by the exchange's parity: a CTA that is one exchange
+// ahead uses the other set, and none can be two ahead.  370 ns on 16 CTAs,
+// all barriers included, where ordinary stores and a releasing arrival take
+// 820 (a grid exchange: 1.3 to 1.8 us).
+//
+// U columns travel the same way: the CTA that owns a column forms it from its
+// own rows of W and stores it into every CTA's coefficient array, completing
+// their `col` barriers.  (Reading W where it lies instead took 1 700 cycles
+// per step: sixteen CTAs at the same few words of one.)
+struct ClusterShared {
+  unsigned long long rec[2][kClusterMax][kClusterWords];
+  unsigned long long bar[2];
+  unsigned long long col[2];
+  int failed;  // a wait on a col barrier ran out
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// the same shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Stores v at a peer's `addr` and completes 8 bytes of its barrier `bar`.
+__device__ __forceinline__ void st_async(uint32_t addr, unsigned long long v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(addr), "l"(v),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void expect_bytes(uint32_t bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Bounded wait for phase `phase` of a barrier in this CTA's shared memory.
+__device__ __forceinline__ bool cluster_wait(const PanelArgs& P, uint32_t bar, uint32_t phase) {
+  unsigned long long t0 = 0;
+  for (unsigned iter = 1;; ++iter) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    if (done) return true;
+    if ((iter & 31u) == 0) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      const bool stop = ld_relaxed_s32(&P.st->abort) != 0;
+      if (stop || now - t0 > P.timeout_ns) {
+        if (!stop) fail(P.st, BBK_ERR_TIMEOUT);
+        return false;
+      }
+    }
+  }
+}
+
+// After a wait ran out: lets stores in flight land, and no CTA leaves while
+// another may still write to it.
+__device__ __forceinline__ void cluster_abandon() {
+  __nanosleep(20000);
+  cluster_barrier();
+}
+
+template <bool kTwo, typename OwnerOf>
+__device__ __forceinline__ XResult cluster_exchange(const PanelArgs& P, int G, unsigned seq, Cand ca, Cand cb,
+                                                    const double* pub_in, OwnerOf&& pub_owner, int npub, XShared& X,
+                                                    ClusterShared& C) {
+  constexpr int kRec = kTwo ? 5 : 2;  // value, index | slot << 32 (twice), payload
+  const int t = threadIdx.x;
+  const int lane = t & 31, warp = t >> 5;
+  const unsigned par = seq & 1u;
+  warp_channel_a<kTwo>(ca);
+  if (kTwo) warp_argmax<true>(cb);
+  if (lane == 0 && warp < kWarps) {
+    X.pa[warp] = ca;
+    if (kTwo) X.pb[warp] = cb;
+  }
+  __syncthreads();
+  const unsigned long long t_stat = P.stats ? globaltimer_ns() : 0;
+  const uint32_t bar = smem_addr(&C.bar[par]);
+  if (t == kThreads) expect_bytes(bar, G * (kRec + npub) * 8);
+  bool ok = C.failed == 0;
+  {
+    // every warp forms the record and sends it to its share of the CTAs
+    Cand a = lane < kWarps ? X.pa[lane] : no_cand();
+    Cand b = kTwo && lane < kWarps ? X.pb[lane] : no_cand();
+    warp_channel_a<kTwo>(a);
+    if (kTwo) warp_argmax<true>(b);
+    auto pack = [](const Cand& c) {
+      return static_cast<unsigned long long>(static_cast<unsigned>(c.i)) |
+             (static_cast<unsigned long long>(static_cast<unsigned>(c.s)) << 32);
+    };
+    unsigned long long word = 0;
+    if (lane == 0) word = static_cast<unsigned long long>(__double_as_longlong(a.v));
+    if (lane == 1) word = pack(a);
+    if (kTwo && lane == 2) word = static_cast<unsigned long long>(__double_as_longlong(b.v));
+    if (kTwo && lane == 3) word = pack(b);
+    if (kTwo && lane == 4) word = static_cast<unsigned long long>(__double_as_longlong(b.pay));
+    if (lane >= kRec && lane < kRec + npub)
+      word = static_cast<unsigned long long>(__double_as_longlong(pub_in[lane - kRec]));
+    if (lane < kRec + npub) {
+      const uint32_t dst = smem_addr(&C.rec[par][blockIdx.x][lane]);
+      for (int k = warp; k < G; k += kAllWarps)
+        st_async(map_rank(dst, k), word, map_rank(bar, k));
+    }
+  }
+  ok = cluster_wait(P, bar, (seq >> 1) & 1u) && ok;
+  if (warp == kCommWarp && lane < npub)
+    X.pub[lane] = __longlong_as_double(static_cast<long long>(C.rec[par][pub_owner(lane)][kRec + lane]));
+  XResult r;
+  r.ok = __syncthreads_and(ok);
+  if (!r.ok) return r;
+  if (P.stats && blockIdx.x == 0 && t == kThreads) atomicAdd(P.stats + 7, globaltimer_ns() - t_stat);
+  // every warp reduces the records, one per lane
+  auto unpack = [&](int k, Cand& c) {
+    const unsigned long long w = C.rec[par][lane][k + 1];
+    c.v = __longlong_as_double(static_cast<long long>(C.rec[par][lane][k]));
+    c.i = static_cast<int>(w & 0xffffffffu);
+    c.s = static_cast<int>(w >> 32);
+  };
+  r.a = no_cand();
+  r.b = no_cand();
+  if (lane < G) {
+    unpack(0, r.a);
+    if (kTwo) {
+      unpack(2, r.b);
+      r.b.pay = __longlong_as_double(static_cast<long long>(C.rec[par][lane][4]));
+    }
+  }
+  warp_channel_a<kTwo>(r.a);
+  if (kTwo) warp_argmax<true>(r.b);
+  return r;
+}
+
+// Gathers the interchanged data (written back by finalize_kernel), by thread
+// gtid of nthreads: each keeps four loads in flight.
+__device__ void gather_moved(const PanelArgs& P, int kstart, long long gtid, long long nthreads) {
+  const int n = P.n;
+  const long long ldw = P.ldw;
+  const int cnt = ldcg(&P.st->moved[P.panel & 1]);
+  if (gtid == 0) P.move_counts[P.panel] = cnt;
+  if (cnt == 0) return;
+  const int* list = P.moved + (P.panel & 1) * P.move_cap;
+  const long long m = n - kstart, total = cnt * m;
+  // rows of the moved indices over the active columns: gbuf[ix][y - k0] = A(src x, src y)
+  for (long long base = gtid; base < total; base += 4 * nthreads) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long idx = base + u * nthreads;
+      v[u] = 0.0;
+      if (idx < total) {
+        const int ix = static_cast<int>(idx / m);
+        const int y = kstart + static_cast<int>(idx - ix * m);
+        const int sx = ldcg(P.srcmap + ldcg(list + ix));
+        const int sy = ldcg(P.srcmap + y);
+        v[u] = __ldg(sx <= sy ? P.a + static_cast<long long>(sx) * P.lda + sy
+                              : P.a + static_cast<long long>(sy) * P.lda + sx);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long idx = base + u * nthreads;
+      if (idx < total) {
+        const int ix = static_cast<int>(idx / m);
+        P.gbuf[ix * ldw + (idx - ix * m)] = v[u];
+      }
+    }
+  }
+  // the moves (position dst receives what position src held): the factored
+  // rows q < k0 take the same column exchanges (:472-491), applied once
+  // after the last panel (launch_left_swaps)
+  int* rec = P.moves + static_cast<size_t>(P.panel) * 2 * P.move_cap;
+  for (long long ix = gtid; ix < cnt; ix += nthreads) {
+    const int x = ldcg(list + ix);
+    rec[ix] = x;
+    rec[P.move_cap + ix] = ldcg(P.srcmap + x);
+    P.permbuf[ix] = ldcg(P.perm + ldcg(P.srcmap + x));
+  }
+}
+
+// f with the number of 32-slot chunks that cover `width` (1..kMax) as a
+// constant, so that sums over them are plain registers and the chunks beyond
+// cost nothing.
+template <int kMax, typename F>
+__device__ __forceinline__ void by_chunks(int width, F&& f) {
+  if constexpr (kMax > 1) {
+    if (width <= 32 * (kMax - 1)) {
+      by_chunks<kMax - 1>(width, f);
+      return;
+    }
+  }
+  f(std::integral_constant<int, kMax>{});
 }
 
 // kOrdered: the row and candidate dot products in the reference's order
 // (bitwise the reference); otherwise reassociated (split_dot).
 // kSmemW: the CTA's panel rows live in shared memory (else in global memory,
 // for orders whose slice does not fit).
-template <bool kOrdered, bool kSmemW>
+// kCluster: the grid is one thread-block cluster.  Exchanges go through the
+// cluster's shared memory, and so do U columns: they are formed from W and
+// the pivots' scaling, which every CTA keeps, by their owner instead of being
+// stored; gather_kernel collects the moved rows afterwards.
+template <bool kOrdered, bool kSmemW, bool kCluster>
 __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
+  static_assert(kSmemW || !kCluster, "a cluster panel keeps its rows in shared memory");
+  constexpr int kPairs = kCluster ? kClusterSlots : kPairSlots;
+  constexpr int kPairLanes = kPairs / 32;
   extern __shared__ double dsm[];
   __shared__ XShared X;
   __shared__ double s_pub[kMaxPub];
+  __shared__ double s_quot[3];  // quotients the communication warp forms for everyone
+  __shared__ __align__(16) unsigned char cluster_smem[kCluster ? sizeof(ClusterShared) : 16];
+  ClusterShared& C = *reinterpret_cast<ClusterShared*>(cluster_smem);
 
   if (ld_relaxed_s32(&P.st->abort)) return;
   const int G = gridDim.x;
@@ -366,16 +611,21 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   const int n = P.n;
   const int kstart = ldcg(&P.st->kstart[P.panel & 1]);
   const int S = (n - kstart + G - 1) / G;  // slots per CTA
-  // reassociated modes with at most kPairSlots slots per CTA: the compute
+  const int SP = kCluster ? (S | 1) : S;   // row pitch of the slice (odd: columns are read without bank conflicts)
+  // reassociated modes with at most kPairs slots per CTA: the compute
   // warps split the rows of the candidate and look-ahead sums
-  const bool paired = !kOrdered && S <= kPairSlots;
+  const bool paired = !kOrdered && S <= kPairs;
   const int lo = kstart + c * S;
   const int hi = min(n, lo + S);
   const int width = max(0, hi - lo);
   const int nwin = min(P.win_rows, n - kstart);  // panel rows staged per slot
   const long long lda = P.lda, ldw = P.ldw;
   const int ldu = P.ldu;
-  auto owner = [&](int z) -> int { return (z - kstart) / S; };
+  // (z - kstart) / S: exact by a multiplication, (z - kstart) S < 2^32
+  const unsigned inv_s = S > 1 ? 0xffffffffu / static_cast<unsigned>(S) + 1u : 0u;
+  auto owner = [&](int z) -> int {
+    return S > 1 ? static_cast<int>(__umulhi(static_cast<unsigned>(z - kstart), inv_s)) : z - kstart;
+  };
   // shared memory: two coefficient columns, candidate column and row computed
   // ahead of this CTA's slots, the per-warp partial sums, the slots' panel
   // rows wsm[m*S + (z - lo)] (all of them, or the first srows), then the maps
@@ -383,20 +633,25 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   double* coef2 = dsm + P.coef_cap;  // coefficients of a row computed ahead
   double* wcs = dsm + 2 * P.coef_cap;
   double* svs = wcs + P.smem_cols;   // the row computed ahead, by slot
-  double* wpart = svs + P.smem_cols;  // per-warp partial sums: 2 x kWarps x kPairSlots
-  double* wsm = wpart + 2 * kWarps * kPairSlots;  // wcap doubles
+  double* wpart = svs + P.smem_cols;  // per-warp partial sums: 2 x kWarps x kPairs
+  double* wsm = wpart + 2 * kWarps * kPairs;  // wcap doubles
   int* win = reinterpret_cast<int*>(wsm + P.wcap);
   int* mypos = win + P.win_pad;  // index held by slot lo + zz
+  // cluster panels: how row q of U follows from W (upk: 1 W / ua; 2 first, 3
+  // second row of a 2x2 pivot, with the coefficients ua, ub of its two rows)
+  double* ua = reinterpret_cast<double*>(mypos + (P.smem_cols + (P.smem_cols & 1)));
+  double* ub = ua + P.coef_cap;
+  int* upk = reinterpret_cast<int*>(ub + P.coef_cap);
   // panel rows kept in shared memory: all of them, or as many rows of this
   // panel's slot width as the allocation holds
   const int srows = kSmemW ? P.win_rows : min(P.win_rows, P.wcap / max(S, 1));
   auto wat = [&](int m, int z) -> double& {
-    if (kSmemW || m < srows) return wsm[m * S + (z - lo)];
+    if (kSmemW || m < srows) return wsm[m * SP + (z - lo)];
     return P.wslot[m * ldw + z];
   };
   // the same, split by where the rows live (the hot dot products run over
   // the shared-memory rows and then the global ones)
-  auto wat_s = [&](int m, int z) -> double { return wsm[m * S + (z - lo)]; };
+  auto wat_s = [&](int m, int z) -> double { return wsm[m * SP + (z - lo)]; };
   auto wat_g = [&](int m, int z) -> double { return P.wslot[m * ldw + z]; };
   // A(x, z) of the symmetric matrix from its upper triangle (A is not written
   // while the panel runs)
@@ -427,16 +682,58 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
     const double* src = x <= z ? P.a + static_cast<long long>(x) * lda + z
                                : P.a + static_cast<long long>(z) * lda + x;
     if (kSmemW || m < srows)
-      cp_async_8(&wsm[m * S + zz], src);
+      cp_async_8(&wsm[m * SP + zz], src);
     else
       P.wslot[m * ldw + z] = __ldg(src);
   }
+  // cluster panels: U[q, x] of this CTA's slot lo + zz, as the scaling phase
+  // of a grid panel would have stored it
+  auto u_value = [&](int zz, int q) -> double {
+    const int kind = upk[q];
+    const double x = wsm[q * SP + zz];
+    if (kind == 1) return div_or_zero(x, ua[q]);
+    if (kind == 2) return xadd(xmul(ua[q], x), xmul(ub[q], wsm[(q + 1) * SP + zz]));
+    return xadd(xmul(ua[q], wsm[(q - 1) * SP + zz]), xmul(ub[q], x));
+  };
+  int cols = 0;  // column transfers so far
+  // U[q, .], q < rows, of `slot` into every CTA's coef, and (slot2 >= 0) of
+  // slot2 into coef2; by every warp, 32 rows at a time
+  auto push_columns = [&](int slot, int slot2, int rows) {
+    if (rows <= 0) return;
+    const uint32_t bar = smem_addr(&C.col[cols & 1]);
+    if (t == kThreads) expect_bytes(bar, rows * (slot2 >= 0 ? 16 : 8));
+    for (int k = 0; k < 2; ++k) {
+      const int z = k == 0 ? slot : slot2;
+      if (z < lo || z >= hi) continue;
+      const uint32_t dst = smem_addr(k == 0 ? coef : coef2);
+      for (int q = t; q < rows; q += kBlock) {
+        const unsigned long long v = static_cast<unsigned long long>(__double_as_longlong(u_value(z - lo, q)));
+        for (int r = 0; r < G; ++r) st_async(map_rank(dst + q * 8, r), v, map_rank(bar, r));
+      }
+    }
+  };
+  // the communication warp waits for them; the others meet it at a CTA barrier
+  auto await_columns = [&](int rows) {
+    if (rows > 0 && t >= kThreads && !cluster_wait(P, smem_addr(&C.col[cols & 1]), (cols >> 1) & 1)) C.failed = 1;
+    if (rows > 0) ++cols;
+  };
+  if (kCluster && t == 0) {
+    C.failed = 0;
+    for (int k = 0; k < 2; ++k) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&C.bar[k])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&C.col[k])) : "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   cp_async_wait_all();
-  __syncthreads();
+  if (kCluster)
+    cluster_barrier();  // every CTA's barriers are ready
+  else
+    __syncthreads();
 
   // exchanges are numbered across the factorization; the k-th (from 1) uses
-  // tag k
-  unsigned seq = static_cast<unsigned>(ldcg(&P.st->xseq[P.panel & 1]));
+  // tag k (a cluster panel numbers its own)
+  unsigned seq = kCluster ? 0u : static_cast<unsigned>(ldcg(&P.st->xseq[P.panel & 1]));
   int p = kstart;
   // coefficients U[q, p] of the current row: rows q < n_old from the Uslot
   // column of p's slot, then lp - n_old (<= 2) values computed by every CTA.
@@ -492,14 +789,16 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         av[k] = v;
       }
       {
-        if (coef_pre) {
+        if (kCluster) {
+          await_columns(n_old);
+        } else if (coef_pre) {
           if (tz < n_old) coef[tz] = cpre[0];
           if (tz + kThreads < n_old) coef[tz + kThreads] = cpre[1];
         } else {
           const double* ucol = P.uslot + static_cast<size_t>(sp) * ldu;
           for (int q = t; q < n_old; q += kBlock) coef[q] = ldcg(ucol + q);
         }
-        if (t == 0) {
+        if (t == kThreads) {
           coef[n_old] = extra0;
           coef[n_old + 1] = extra1;
         }
@@ -507,7 +806,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       }
       __syncthreads();
       // release the previous steps' U rows while the compute warps update the row
-      if (t == kThreads) fence_acq_rel_gpu();
+      if (!kCluster && t == kThreads) fence_acq_rel_gpu();
       Cand best = no_cand();
       auto finish_row = [&](int z, int j, double a_val, double acc) {
         const double wv = xsub(a_val, acc);
@@ -524,34 +823,37 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         if (t < kThreads) {
           const int w = t >> 5, ln = t & 31;
           const int qa = (lp * w) / kWarps, qb = (lp * (w + 1)) / kWarps;
-          double s1[3] = {0.0, 0.0, 0.0};
-          auto rows = [&](int q0, int q1, auto&& wget) {
-            for (int q = q0; q < q1; ++q) {
-              const double c1 = coef[q];
-#pragma unroll
-              for (int k = 0; k < 3; ++k) {
-                const int zz = ln + 32 * k;
-                if (zz < width) s1[k] = __fma_rn(c1, wget(q, lo + zz), s1[k]);
-              }
-            }
-          };
           const int qm = kSmemW ? qb : min(max(qa, srows), qb);
-          rows(qa, qm, wat_s);
-          if (!kSmemW) rows(qm, qb, wat_g);
+          by_chunks<kPairLanes>(width, [&](auto chunks) {
+            constexpr int N = decltype(chunks)::value;
+            double s1[N] = {};
+            auto rows = [&](int q0, int q1, const double* wp, long long pitch) {
+              for (int q = q0; q < q1; ++q, wp += pitch) {
+                const double c1 = coef[q];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const int zz = ln + 32 * k;
-            if (zz < width) wpart[w * kPairSlots + zz] = s1[k];
-          }
+                for (int k = 0; k < N; ++k)
+                  if (k < N - 1 || ln + 32 * k < width) s1[k] = __fma_rn(c1, wp[32 * k], s1[k]);
+              }
+            };
+            rows(qa, qm, wsm + qa * SP + ln, SP);
+            if (!kSmemW) rows(qm, qb, P.wslot + qm * ldw + lo + ln, ldw);
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+              if (k < N - 1 || ln + 32 * k < width) wpart[w * kPairs + ln + 32 * k] = s1[k];
+          });
           compute_warps_sync();
         }
-        if (t < width) {
-          const int j = mypos[t];
-          if (j >= p) {
-            double acc = wpart[t];
 #pragma unroll
-            for (int w = 1; w < kWarps; ++w) acc += wpart[w * kPairSlots + t];
-            finish_row(lo + t, j, av[0], acc);
+        for (int k = 0; k < (kPairs + kThreads - 1) / kThreads; ++k) {
+          const int zz = tz + k * kThreads;
+          if (zz < width) {
+            const int j = mypos[zz];
+            if (j >= p) {
+              double acc = wpart[zz];
+#pragma unroll
+              for (int w = 1; w < kWarps; ++w) acc += wpart[w * kPairs + zz];
+              finish_row(lo + zz, j, av[k], acc);
+            }
           }
         }
       } else {
@@ -578,12 +880,16 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         }
       }
       lap(0);
-      int owners[kMaxPub] = {};
-      owners[0] = owner(sp);
-      owners[1] = lp + 1 < nwin ? owner(win[lp + 1]) : 0;
-      owners[2] = lp + 2 < nwin ? owner(win[lp + 2]) : 0;
-      const XResult x1 = exchange<false>(P, ++seq, false, best, no_cand(), s_pub, owners, 3, X);
-      if (!x1.ok) return;
+      // published by the CTAs that own W[p, p], W[p, p+1], W[p, p+2]
+      auto owner_of = [&](int k) { return lp + k < nwin ? owner(win[lp + k]) : 0; };
+      ++seq;
+      const XResult x1 = kCluster
+                             ? cluster_exchange<false>(P, G, seq - 1, best, no_cand(), s_pub, owner_of, 3, X, C)
+                             : exchange<false>(P, seq, false, best, no_cand(), s_pub, owner_of, 3, X);
+      if (!x1.ok) {
+        if (kCluster) cluster_abandon();
+        return;
+      }
       omega = x1.a.v;
       r = x1.a.i;
       rs = x1.a.s;  // slot of r
@@ -605,7 +911,8 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
     // the rest of the step: A = slot of p+1, B = slot of p+2 (2x2 pivot),
     // C = slot of p (r = p+1).  After a row computed ahead, A (and the
     // candidate's operands) were loaded by the previous step.
-    const bool prefetch = lp <= 2 * kThreads;
+    // (a cluster panel forms them when they are needed)
+    const bool prefetch = !kCluster && lp <= 2 * kThreads;
     auto preload = [&](int slot, int rows, double& c0, double& c1) {
       const double* ucol = P.uslot + static_cast<size_t>(slot) * ldu;
       c0 = tz < rows ? ldcg(ucol + tz) : 0.0;
@@ -658,21 +965,32 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
           coef2[tz + kThreads] = ca1;
         }
       } else {
-        const double* ucol = P.uslot + static_cast<size_t>(rs) * ldu;
-        for (int q = t; q < nrel; q += kBlock) coef[q] = ldcg(ucol + q);
-        if (spec) {
-          const double* ucol2 = P.uslot + static_cast<size_t>(slot_a) * ldu;
-          for (int q = t; q < nrel; q += kBlock) coef2[q] = ldcg(ucol2 + q);
+        if (kCluster) {
+          // after a row computed ahead they are on their way already
+          if (!was_ahead) push_columns(rs, spec ? slot_a : -1, nrel);
+          await_columns(nrel);
+        } else {
+          const double* ucol = P.uslot + static_cast<size_t>(rs) * ldu;
+          for (int q = t; q < nrel; q += kBlock) coef[q] = ldcg(ucol + q);
+          if (spec) {
+            const double* ucol2 = P.uslot + static_cast<size_t>(slot_a) * ldu;
+            for (int q = t; q < nrel; q += kBlock) coef2[q] = ldcg(ucol2 + q);
+          }
         }
       }
-      if (was_ahead && t == 0) {
+      if (was_ahead && t == kThreads) {
         coef[lp - 1] = u_prev_r;
         coef2[lp - 1] = carry;
+      }
+      // U[p, p+1] if p stays a 1x1 pivot (after a row computed ahead it is there)
+      if (spec && !was_ahead && t >= kThreads) {
+        const double u = div_or_zero(w_p1, safe_denominator(dpp));
+        if (t == kThreads) s_quot[0] = u;
       }
       if (t < kMaxPub) s_pub[t] = 0.0;
       __syncthreads();
       // release U row lp - 1 (written by the previous step, after its last exchange)
-      if (was_ahead && t == kThreads) fence_acq_rel_gpu();
+      if (!kCluster && was_ahead && t == kThreads) fence_acq_rel_gpu();
       // ---- candidate column W(i, r) = A(i, r) - sum_q U[q, r] W[q, i]
       // (CopyCandidateToWorkspace + UpdateCandidateInWorkspace, :184-352), and
       // row p+1 as keeping pivot p leaves it: W[p+1, j] = A(p+1, j) -
@@ -680,7 +998,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       // W[lp, r] becomes the candidate's W(p, r), so the owner publishes
       // A(p+1, r) and the partial sum instead.
       const bool staged1 = spec && (slot_a - kstart) == lp + 1;
-      if (spec) e0 = div_or_zero(w_p1, safe_denominator(dpp));
+      if (spec) e0 = s_quot[0];
       Cand best = no_cand();
       double sig = 0.0;
       // slot z holding index i >= p, with its candidate sum acc and (two) the
@@ -723,44 +1041,47 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         if (t < kThreads) {
           const int w = t >> 5, ln = t & 31;
           const int qa = (lp * w) / kWarps, qb = (lp * (w + 1)) / kWarps;
-          double sa[3] = {0.0, 0.0, 0.0}, sb[3] = {0.0, 0.0, 0.0};
-          auto rows = [&](int q0, int q1, auto&& wget) {
-            for (int q = q0; q < q1; ++q) {
-              const double c1 = coef[q], c2 = coef2[q];
-#pragma unroll
-              for (int k = 0; k < 3; ++k) {
-                const int zz = ln + 32 * k;
-                if (zz < width) {
-                  const double x = wget(q, lo + zz);
-                  sa[k] = __fma_rn(c1, x, sa[k]);
-                  sb[k] = __fma_rn(c2, x, sb[k]);
-                }
-              }
-            }
-          };
           const int qm = kSmemW ? qb : min(max(qa, srows), qb);
-          rows(qa, qm, wat_s);
-          if (!kSmemW) rows(qm, qb, wat_g);
+          by_chunks<kPairLanes>(width, [&](auto chunks) {
+            constexpr int N = decltype(chunks)::value;
+            double sa[N] = {}, sb[N] = {};
+            auto rows = [&](int q0, int q1, const double* wp, long long pitch) {
+              for (int q = q0; q < q1; ++q, wp += pitch) {
+                const double c1 = coef[q], c2 = coef2[q];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const int zz = ln + 32 * k;
-            if (zz < width) {
-              wpart[(2 * w) * kPairSlots + zz] = sa[k];
-              wpart[(2 * w + 1) * kPairSlots + zz] = sb[k];
-            }
-          }
+                for (int k = 0; k < N; ++k)
+                  if (k < N - 1 || ln + 32 * k < width) {
+                    const double x = wp[32 * k];
+                    sa[k] = __fma_rn(c1, x, sa[k]);
+                    sb[k] = __fma_rn(c2, x, sb[k]);
+                  }
+              }
+            };
+            rows(qa, qm, wsm + qa * SP + ln, SP);
+            if (!kSmemW) rows(qm, qb, P.wslot + qm * ldw + lo + ln, ldw);
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+              if (k < N - 1 || ln + 32 * k < width) {
+                wpart[(2 * w) * kPairs + ln + 32 * k] = sa[k];
+                wpart[(2 * w + 1) * kPairs + ln + 32 * k] = sb[k];
+              }
+          });
           compute_warps_sync();
         }
-        if (t < width) {
-          const int i = mypos[t];
-          if (i >= p) {
-            double acc = wpart[t], part = wpart[kPairSlots + t];
 #pragma unroll
-            for (int w = 1; w < kWarps; ++w) {
-              acc += wpart[(2 * w) * kPairSlots + t];
-              part += wpart[(2 * w + 1) * kPairSlots + t];
+        for (int k = 0; k < (kPairs + kThreads - 1) / kThreads; ++k) {
+          const int zz = tz + k * kThreads;
+          if (zz < width) {
+            const int i = mypos[zz];
+            if (i >= p) {
+              double acc = wpart[zz], part = wpart[kPairs + zz];
+#pragma unroll
+              for (int w = 1; w < kWarps; ++w) {
+                acc += wpart[(2 * w) * kPairs + zz];
+                part += wpart[(2 * w + 1) * kPairs + zz];
+              }
+              finish(lo + zz, i, acc, part, spec && i > p);
             }
-            finish(lo + t, i, acc, part, spec && i > p);
           }
         }
       } else {
@@ -812,21 +1133,22 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       }
       nx_best = best;
       lap(2);
-      int owners[kMaxPub] = {};
-      owners[0] = owner(rs);
-      owners[1] = owner(sp);
-      owners[2] = lp + 1 < nwin ? owner(win[lp + 1]) : 0;
-      owners[3] = lp + 2 < nwin ? owner(win[lp + 2]) : 0;
-      if (spec) {
-        owners[4] = owner(slot_a);
-        owners[5] = owners[3];
-        owners[6] = lp + 3 < nwin ? owner(win[lp + 3]) : 0;
-        owners[7] = owners[0];
-        owners[8] = owners[0];
+      // published by the owners of r (0, 7, 8), p (1), p+1 (2, 4), p+2 (3, 5)
+      // and p+3 (6)
+      auto owner_of = [&](int k) {
+        if (k == 0 || k >= 7) return owner(rs);
+        const int m = lp + (k < 4 ? k - 1 : k - 3);
+        return m < nwin ? owner(win[m]) : 0;
+      };
+      ++seq;
+      const XResult x2 =
+          kCluster ? cluster_exchange<true>(P, G, seq - 1, Cand{sig, 0, 0, 0.0}, nx_best, s_pub, owner_of, spec ? 9 : 4,
+                                            X, C)
+                   : exchange<true>(P, seq, false, Cand{sig, 0, 0, 0.0}, nx_best, s_pub, owner_of, spec ? 9 : 4, X);
+      if (!x2.ok) {
+        if (kCluster) cluster_abandon();
+        return;
       }
-      const XResult x2 = exchange<true>(P, ++seq, false, Cand{sig, 0, 0, 0.0}, nx_best, s_pub, owners,
-                                        spec ? 9 : 4, X);
-      if (!x2.ok) return;
       const double sigma = x2.a.v;
       wc_r = X.pub[0];
       wc_p = X.pub[1];
@@ -871,6 +1193,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       const double d = dpp;
       const double den = safe_denominator(d);
       double wr = 0.0;  // W[p+1, r] of the row computed ahead
+      double nx_pay = 0.0;  // W[p, r'] of the next step's candidate r'
       if (spec) {
         wr = xsub(nx_ar, xadd(nx_part, xmul(e0, wc_p)));
         // the next step starts from row p+1 and its argmax
@@ -882,8 +1205,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         nx_dpp = nx_d;
         nx_w1 = r == p + 2 ? wr : nx_1;
         nx_w2 = r == p + 3 ? wr : nx_2;
-        u_prev_r = div_or_zero(best.pay, den);
-        carry = div_or_zero(r == p + 2 ? wc_p : w_p2, den);
+        nx_pay = best.pay;
         ahead = true;
         // the next step's operands load while this step scales: its next
         // row's coefficient column (slot of p+2) and, when it evaluates a
@@ -905,25 +1227,38 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
             } else {
               wv = wat(lp, z);
             }
-            P.uslot[static_cast<size_t>(z) * ldu + lp] = div_or_zero(wv, den);
+            if (!kCluster) P.uslot[static_cast<size_t>(z) * ldu + lp] = div_or_zero(wv, den);
             if (spec) wat(lp + 1, z) = j == r ? wr : svs[z - lo];
           }
         }
+      }
+      if (kCluster && t == 0) {
+        upk[lp] = 1;
+        ua[lp] = den;
       }
       if (c == 0 && t == 0) {
         P.dlog[2 * lp] = d;
         P.ptype[p] = 1;
       }
-      if (was_ahead && !cand) {
-        // next row's coefficients: U[q, p+1] for q < lp - 1, then U[lp - 1, p+1]
-        // (passed along) and U[p, p+1]
-        n_old = lp - 1;
-        extra0 = carry;
-        extra1 = div_or_zero(w_p1, den);
-      } else {
-        // next row's coefficients: U[q, p+1] for q < p, then U[p, p+1]
-        n_old = lp;
-        extra0 = div_or_zero((cand && r == p + 1) ? wc_p : w_p1, den);
+      // Next row's coefficients: U[q, p+1] for q < p, then U[p, p+1]; after a
+      // row computed ahead that needed no candidate, U[q, p+1] for q < lp - 1,
+      // then U[lp - 1, p+1] (passed along) and U[p, p+1].
+      n_old = was_ahead && !cand ? lp - 1 : lp;
+      if (t >= kThreads) {
+        // the communication warp divides while the others scale, one quotient
+        // per lane: after this step a row computed ahead needs U[p, r'],
+        // U[p, p+2] and its own U[p+1, p+2]; else the next row U[p, p+1]
+        const int ln = t & 31;
+        const double num = spec ? (ln == 0 ? nx_pay : ln == 1 ? (r == p + 2 ? wc_p : w_p2) : nx_w1)
+                                : ((cand && r == p + 1) ? wc_p : w_p1);
+        const double quot = div_or_zero(num, spec && ln >= 2 ? safe_denominator(nx_dpp) : den);
+        const double q0 = __shfl_sync(0xffffffffu, quot, 0);
+        const double q1 = __shfl_sync(0xffffffffu, quot, 1);
+        if (ln == 2) s_quot[0] = quot;
+        extra0 = was_ahead && !cand ? carry : q0;
+        extra1 = q0;
+        u_prev_r = q0;
+        carry = q1;
       }
       p += 1;
     } else if (kind == -1) {
@@ -944,15 +1279,19 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         if (z < hi && mypos[z - lo] > p) {
           const double wv = wcs[z - lo];
           wat(lp, z) = wv;
-          P.uslot[static_cast<size_t>(z) * ldu + lp] = div_or_zero(wv, den);
+          if (!kCluster) P.uslot[static_cast<size_t>(z) * ldu + lp] = div_or_zero(wv, den);
         }
+      }
+      if (kCluster && t == 0) {
+        upk[lp] = 1;
+        ua[lp] = den;
       }
       if (c == 0 && t == 0) {
         P.dlog[2 * lp] = d;
         P.ptype[p] = 1;
       }
       n_old = lp;
-      extra0 = div_or_zero((r == p + 1) ? wc_p : wc_p1, den);
+      if (t >= kThreads) extra0 = div_or_zero((r == p + 1) ? wc_p : wc_p1, den);
       p += 1;
     } else {
       // SwapTwoByTwoPivot (:403-412, :500-587) + ScaleTwoByTwoPivot (:658-704):
@@ -961,10 +1300,12 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       const int ss = win[ls];
       const double d11 = dpp, d21 = wc_p, d22 = wc_r;
       const double det = xsub(xmul(d11, d22), xmul(d21, d21));
-      const double i11 = xdiv(d22, det);
-      const double i22 = xdiv(d11, det);
-      const double i21 = xdiv(-d21, det);
       __syncthreads();  // every thread has read win[ls]
+      if (t >= kThreads) {  // one quotient per lane
+        const int ln = t & 31;
+        const double quot = xdiv(ln == 0 ? d22 : ln == 1 ? d11 : -d21, det);
+        if (ln < 3) s_quot[ln] = quot;
+      }
       if (r != p + 1 && t == 0) {
         win[ls] = rs;
         if (r - kstart < nwin) win[r - kstart] = ss;
@@ -972,6 +1313,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         if (rs >= lo && rs < hi) mypos[rs - lo] = p + 1;
       }
       __syncthreads();
+      const double i11 = s_quot[0], i22 = s_quot[1], i21 = s_quot[2];
 #pragma unroll
       for (int k = 0; k < kCols; ++k) {
         const int z = lo + tz + k * kThreads;
@@ -979,9 +1321,19 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
           const double x = wat(lp, z);
           const double y = wcs[z - lo];
           wat(ls, z) = y;
-          P.uslot[static_cast<size_t>(z) * ldu + lp] = xadd(xmul(i11, x), xmul(i21, y));
-          P.uslot[static_cast<size_t>(z) * ldu + ls] = xadd(xmul(i21, x), xmul(i22, y));
+          if (!kCluster) {
+            P.uslot[static_cast<size_t>(z) * ldu + lp] = xadd(xmul(i11, x), xmul(i21, y));
+            P.uslot[static_cast<size_t>(z) * ldu + ls] = xadd(xmul(i21, x), xmul(i22, y));
+          }
         }
+      }
+      if (kCluster && t == 0) {
+        upk[lp] = 2;
+        ua[lp] = i11;
+        ub[lp] = i21;
+        upk[ls] = 3;
+        ua[ls] = i21;
+        ub[ls] = i22;
       }
       if (c == 0 && t == 0) {
         P.dlog[2 * lp] = d11;
@@ -997,6 +1349,16 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       extra0 = xadd(xmul(i11, x), xmul(i21, y));
       extra1 = xadd(xmul(i21, x), xmul(i22, y));
       p += 2;
+    }
+    if (kCluster && p < P.nominal_end) {
+      // the next step's coefficients set out: the candidate's and the next
+      // row's columns after a row computed ahead that will evaluate one
+      // (rows before lp), else the next row's
+      if (!ahead)
+        push_columns(win[p - kstart], -1, n_old);
+      else if (!(fabs(nx_dpp) >= xmul(kAlpha, nx_omega) || nx_omega == 0.0))
+        push_columns(nx_rs,
+                     nx_r != p + 1 && p + 1 < P.nominal_end && p + 1 - kstart < nwin ? win[p + 1 - kstart] : -1, lp);
     }
     coef_pre = prefetch && p < P.nominal_end && !ahead;
     if (coef_pre) {
@@ -1034,7 +1396,13 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   __syncthreads();
   for (int idx = t; idx < width * kb; idx += kBlock) {
     const int zz = idx / kb, q = idx - zz * kb;
-    P.ucm[static_cast<size_t>(mypos[zz]) * ldu + q] = P.uslot[static_cast<size_t>(lo + zz) * ldu + q];
+    double u;
+    if (kCluster) {
+      u = u_value(zz, q);
+    } else {
+      u = P.uslot[static_cast<size_t>(lo + zz) * ldu + q];
+    }
+    P.ucm[static_cast<size_t>(mypos[zz]) * ldu + q] = u;
   }
   for (int idx = t; idx < width * kb; idx += kBlock) {
     const int q = idx / width, zz = idx - q * width;
@@ -1052,7 +1420,8 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   if (c == 0 && t == 0) {
     // panel range [kstart, e); the next panel starts at e.
     P.st->kstart[(P.panel + 1) & 1] = e;
-    P.st->xseq[(P.panel + 1) & 1] = static_cast<int>(seq + 1);  // + the barrier below
+    // + the barrier below; a cluster panel leaves the grid's numbers as they are
+    P.st->xseq[(P.panel + 1) & 1] = kCluster ? ldcg(&P.st->xseq[P.panel & 1]) : static_cast<int>(seq + 1);
     if (P.panel_end) P.panel_end[P.panel] = e;
     P.bounds[2 * P.panel] = kstart;
     P.bounds[2 * P.panel + 1] = e;
@@ -1063,39 +1432,24 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
       atomicAdd(P.stats + 9, static_cast<unsigned long long>(nahead));
     }
   }
+  if (kCluster) {
+    cluster_barrier();  // no CTA leaves while another may read its shared memory
+    return;
+  }
   // grid barrier: every CTA's maps and lists are visible after it
   {
-    const int owners0[kMaxPub] = {};
-    const XResult xb = exchange<false>(P, ++seq, true, no_cand(), no_cand(), s_pub, owners0, 0, X);
+    const XResult xb =
+        exchange<false>(P, ++seq, true, no_cand(), no_cand(), s_pub, [](int) { return 0; }, 0, X);
     if (!xb.ok) return;
   }
-  // ---- gather the interchanged data (written back by finalize_kernel)
-  const int cnt = ldcg(&P.st->moved[P.panel & 1]);
-  if (c == 0 && t == 0) P.move_counts[P.panel] = cnt;
-  if (cnt == 0) return;
-  const int* list = P.moved + (P.panel & 1) * P.move_cap;
-  const long long m = n - kstart;
-  const long long nthreads = static_cast<long long>(G) * kBlock;
-  const long long gtid = static_cast<long long>(c) * kBlock + t;
-  // rows of the moved indices over the active columns: gbuf[ix][y - k0] = A(src x, src y)
-  for (long long idx = gtid; idx < cnt * m; idx += nthreads) {
-    const int ix = static_cast<int>(idx / m);
-    const int y = kstart + static_cast<int>(idx - ix * m);
-    const int sx = ldcg(P.srcmap + ldcg(list + ix));
-    const int sy = ldcg(P.srcmap + y);
-    P.gbuf[ix * ldw + (y - kstart)] = asym(sx, sy);
-  }
-  // the moves (position dst receives what position src held): the factored
-  // rows q < k0 take the same column exchanges (:472-491), applied once
-  // after the last panel (launch_left_swaps)
-  int* rec = P.moves + static_cast<size_t>(P.panel) * 2 * P.move_cap;
-  for (long long ix = gtid; ix < cnt; ix += nthreads) {
-    const int x = ldcg(list + ix);
-    rec[ix] = x;
-    rec[P.move_cap + ix] = ldcg(P.srcmap + x);
-  }
-  for (long long ix = gtid; ix < cnt; ix += nthreads)
-    P.permbuf[ix] = ldcg(P.perm + ldcg(P.srcmap + ldcg(list + ix)));
+  gather_moved(P, kstart, static_cast<long long>(c) * kBlock + t, static_cast<long long>(G) * kBlock);
+}
+
+// The gather of a cluster panel, on the whole GPU: with the cluster's CTAs
+// alone it would take as long as a dozen pivot steps.
+__global__ void __launch_bounds__(256) gather_kernel(PanelArgs P) {
+  if (ld_relaxed_s32(&P.st->abort)) return;
+  gather_moved(P, ldcg(&P.st->kstart[P.panel & 1]), blockIdx.x * 256ll + threadIdx.x, gridDim.x * 256ll);
 }
 
 // Writes back what the panel's interchanges moved, the permutation, and the
@@ -1322,13 +1676,12 @@ __global__ void __launch_bounds__(kBlock) probe_kernel(PanelArgs P) {
   __shared__ XShared X;
   __shared__ double s_pub[kMaxPub];
   if (threadIdx.x < kMaxPub) s_pub[threadIdx.x] = 0.0;
-  const int owners[kMaxPub] = {};
   __syncthreads();
   const unsigned long long t0 = globaltimer_ns();
   for (int it = 0; it < P.n; ++it) {
     const Cand mine{static_cast<double>(blockIdx.x), static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.x), 0.0};
     const XResult x = exchange<false>(P, static_cast<unsigned>(it) + 1u, true, mine, no_cand(), s_pub,
-                                      owners, 3, X);
+                                      [](int) { return 0; }, 3, X);
     if (!x.ok) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && P.stats) P.stats[0] = globaltimer_ns() - t0;
@@ -1369,6 +1722,100 @@ int launch_init(int n, int* perm, int* pivot_types, DeviceState* st, unsigned lo
   init_kernel<<<256, 256, 0, s>>>(n, perm, pivot_types, st, slots, slot_words);
   BBK_CUDA_TRY(cudaGetLastError());
   count_launch();
+  return BBK_OK;
+}
+
+constexpr int kClusterCols = 64;  // active columns per CTA that a cluster grows for
+constexpr size_t kClusterSmem = 216 * 1024;
+
+// CTAs of the largest cluster of panel kernels that this device can hold
+// (0: none).
+static int cluster_limit(const void* fn) {
+  static std::mutex mu;
+  static int limit[2][64] = {};  // by kernel and device; 0: not asked yet, -1: none
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int& l = limit[fn == reinterpret_cast<const void*>(panel_kernel<true, true, true>)][dev];
+  std::lock_guard<std::mutex> lk(mu);
+  if (l == 0) {
+    l = -1;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kClusterSmem)) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      for (int g = kClusterMax; g >= 1 && l < 0; g /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(g);
+        cfg.blockDim = dim3(kBlock);
+        cfg.dynamicSmemBytes = kClusterSmem;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = g;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0) l = g;
+      }
+    }
+    cudaGetLastError();  // a refused size is not an error of the call that asks
+  }
+  return std::max(l, 0);
+}
+
+// Launches the panel as one cluster where its active columns fit sixteen
+// CTAs: at most kClusterSlots each, with all panel rows in shared memory
+// (block 64: 3 584 columns, 128: about 3 000, 256: 1 500).  Its exchanges
+// cost a quarter of a grid's, and up to the limit that outweighs the longer
+// slices (panel ms per factorization, cluster up to 0 / 64 / 128 / 224 slots:
+// KKT n = 1999, block 64: 8.56 / 7.75 / 6.90 / 6.90; KKT n = 10000, block
+// 128: 46.2 / 45.4 / 44.7 / 44.4).  The cluster doubles once its CTAs would hold
+// more than kClusterCols (24 to 128 measured within 5 %).
+static int launch_cluster_panel(const FactorPlan& plan, PanelArgs P, bool ordered, bool* launched, cudaStream_t s) {
+  *launched = false;
+  if (getenv("BBK_PANEL_SMEM_ROWS") != nullptr) return BBK_OK;  // the split layout is the grid panel's
+  // at most this many active columns (a boundary shift starts a panel one row early)
+  const long long start = std::max(0LL, static_cast<long long>(P.panel) * plan.b - 1);
+  const long long m = plan.n - start;
+  if (m > static_cast<long long>(kClusterMax) * kClusterSlots) return BBK_OK;
+  const void* fn = ordered ? reinterpret_cast<const void*>(panel_kernel<true, true, true>)
+                           : reinterpret_cast<const void*>(panel_kernel<false, true, true>);
+  int G = 1;
+  while (G < kClusterMax && m > static_cast<long long>(kClusterCols) * G) G *= 2;
+  G = std::min(G, cluster_limit(fn));
+  if (G < 1) return BBK_OK;
+  const long long smax = (m + G - 1) / G;
+  if (smax > kClusterSlots) return BBK_OK;
+  P.coef_cap = static_cast<int>(align_up(static_cast<size_t>(plan.b) + 4, 2));
+  P.smem_cols = static_cast<int>(smax);
+  P.w_smem = 1;
+  P.wcap = P.win_rows * static_cast<int>(smax | 1);
+  const size_t cols = align_up(static_cast<size_t>(smax), 2);
+  const size_t bytes = (4 * static_cast<size_t>(P.coef_cap) + 2 * static_cast<size_t>(smax) +
+                        2 * static_cast<size_t>(kWarps) * kClusterSlots + P.wcap) * sizeof(double) +
+                       (2 * static_cast<size_t>(P.win_pad) + cols) * sizeof(int);
+  if (bytes > kClusterSmem) return BBK_OK;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(G);
+  cfg.blockDim = dim3(kBlock);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = G;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  void* kargs[] = {&P};
+  cudaError_t err = cudaLaunchKernelExC(&cfg, fn, kargs);
+  if (err != cudaSuccess) return cuda_error(err, "cudaLaunchKernelEx(panel)");
+  const long long work = 2LL * plan.b * m;
+  gather_kernel<<<static_cast<int>(std::max(1LL, std::min(4LL * device_sm_count(), (work + 1023) / 1024))), 256, 0,
+                  s>>>(P);
+  BBK_CUDA_TRY(cudaGetLastError());
+  count_launch(2);
+  *launched = true;
   return BBK_OK;
 }
 
@@ -1418,6 +1865,12 @@ int launch_panel(const FactorPlan& plan, int panel, cudaStream_t s) {
   // shared memory: two coefficient columns + candidate column + row computed
   // ahead + per-warp partial sums + the slots' panel rows (all, or as many
   // as fit), then the window map and the slot -> index map
+  const bool ordered = plan.mode == BBK_UPDATE_FP64_ORDERED;
+  bool clustered = false;
+  {
+    const int rc = launch_cluster_panel(plan, P, ordered, &clustered, s);
+    if (rc || clustered) return rc;
+  }
   const int smax = (plan.n + plan.grid - 1) / plan.grid;
   P.coef_cap = static_cast<int>(align_up(static_cast<size_t>(plan.b) + 4, 2));
   P.smem_cols = smax;
@@ -1443,11 +1896,10 @@ int launch_panel(const FactorPlan& plan, int panel, cudaStream_t s) {
   }
   P.wcap = static_cast<int>(wroom / sizeof(double));
   const size_t bytes = base + wroom;
-  const bool ordered = plan.mode == BBK_UPDATE_FP64_ORDERED;
-  const void* fn = ordered ? (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<true, true>)
-                                       : reinterpret_cast<const void*>(panel_kernel<true, false>))
-                           : (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<false, true>)
-                                       : reinterpret_cast<const void*>(panel_kernel<false, false>));
+  const void* fn = ordered ? (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<true, true, false>)
+                                       : reinterpret_cast<const void*>(panel_kernel<true, false, false>))
+                           : (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<false, true, false>)
+                                       : reinterpret_cast<const void*>(panel_kernel<false, false, false>));
   BBK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
   void* kargs[] = {&P};
   cudaError_t err = cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(kBlock), kargs, bytes, s);

@@ -1,0 +1,76 @@
+"""GPU: panels on one thread-block cluster (up to 3584 active columns).  In
+the ordered mode the factors are the oracle's bit for bit, in the FP64 mode
+the pivots are and the residual is within the reference's 1e-10; at the
+orders where the cluster grows (64 columns per CTA), where the first panels
+run on the grid and the last ones on a cluster, and with panels wider than a
+cluster's shared memory takes."""
+import numpy as np
+import pytest
+
+from common import kkt_matrix, reconstruct, relative_error, uniform_symmetric
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(1, 1), (2, 1), (3, 2), (64, 16), (65, 16), (66, 64), (129, 32), (257, 31), (513, 48), (1025, 64),
+         (1300, 255),  # the first panel's rows do not fit a cluster
+         (700, 350), (2049, 100)]
+
+
+def _check(bbk, cuda, a, b, mode, want):
+    import torch
+    f = torch.from_numpy(a).to(cuda)
+    perm, pt, ends = bbk.factor_device(f, b, mode=mode)
+    assert np.array_equal(pt.cpu().numpy(), want.pivot_types)
+    assert np.array_equal(perm.cpu().numpy(), want.perm)
+    assert np.array_equal(ends.cpu().numpy(), want.panel_end)
+    return np.triu(f.cpu().numpy()), perm.cpu().numpy(), pt.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,b", CASES)
+@pytest.mark.parametrize("kind", ["random", "kkt"])
+def test_cluster_panels_are_the_oracles(cuda, bbk, port, n, b, kind):
+    a = kkt_matrix(n, max(1, (3 * n) // 4), n + b) if kind == "kkt" else uniform_symmetric(n, n + b)
+    want = port.factor(a, b)
+    f, _, _ = _check(bbk, cuda, a, b, "fp64_ordered", want)
+    assert np.array_equal(f, np.triu(want.factors), equal_nan=True)
+    f, perm, pt = _check(bbk, cuda, a, b, "fp64", want)
+    if n <= 700:
+        assert relative_error(reconstruct(f, perm, pt), a) < 1e-10
+
+
+def test_grid_panels_then_cluster_panels(cuda, bbk, port):
+    n, b = 3650, 64  # 3 584 columns are active at the second panel
+    a = uniform_symmetric(n, 8)
+    want = port.factor(a, b)
+    f, _, _ = _check(bbk, cuda, a, b, "fp64_ordered", want)
+    assert np.array_equal(f, np.triu(want.factors), equal_nan=True)
+    _check(bbk, cuda, a, b, "fp64", want)
+
+
+@pytest.mark.parametrize("value", [0.0, np.nan, np.inf])
+def test_cluster_panels_with_degenerate_entries(cuda, bbk, port, value):
+    n, b = 300, 32
+    a = uniform_symmetric(n, 4)
+    a[40:90, :] = a[:, 40:90] = 0.0  # zero rows: zero pivots
+    a[10, 200] = a[200, 10] = value
+    a[250, 250] = value
+    want = port.factor(a, b)
+    f, _, _ = _check(bbk, cuda, a, b, "fp64_ordered", want)
+    assert np.array_equal(f, np.triu(want.factors), equal_nan=True)
+
+
+def test_an_expired_wait_in_a_cluster_is_reported_and_the_context_survives(cuda, bbk):
+    import torch
+    a = uniform_symmetric(900, 3)
+    bbk.set_wait_timeout_ns(1)
+    try:
+        try:
+            bbk.factor_device(torch.from_numpy(a).to(cuda), 64)
+        except bbk.BbkError as e:
+            assert e.status == bbk.BBK_ERR_TIMEOUT
+    finally:
+        bbk.set_wait_timeout_ns(5_000_000_000)
+    f = torch.from_numpy(a).to(cuda)
+    perm, pt, _ = bbk.factor_device(f, 64)
+    r = bbk.reconstruct_device(f, perm, pt).cpu().numpy()
+    assert relative_error(r, a) < 1e-10
