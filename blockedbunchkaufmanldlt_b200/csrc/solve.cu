@@ -9,15 +9,14 @@
 //   y = B[perm]; L z = y; D w = z; L^T v = w; X[perm] = v.
 // Each triangular sweep is a persistent cooperative launch over 64-row
 // blocks in sweep order: CTA c owns blocks c, c+G, ...; a solved block is
-// published with a release flag.  Two forms:
-//  * pull (up to 32 right-hand sides, 8 per launch): the owner of a block
-//    gathers the contributions of all earlier blocks into it, the old ones
-//    while the blocks just before it are still being solved elsewhere, then
-//    solves its triangle.  The critical path per block is one flag, one fold
-//    and the triangle.
-//  * streaming (more right-hand sides): every solved block is pushed into
-//    each later block of every CTA, all right-hand sides at once, so the
-//    factor is read once per sweep.
+// published with a release flag.  The owner of a block gathers the
+// contributions of all earlier blocks into it, the old ones while the blocks
+// just before it are still being solved elsewhere, then solves its triangle
+// with inverses it formed meanwhile.  The critical path per block is one
+// flag, one fold and three 32 x 32 products.  Right-hand sides go in groups
+// of eight, up to sixteen groups side by side on CTAs of their own.
+// Measured: n = 10000, 1 right-hand side: 1.74 -> 1.34 ms (4.3 us per block);
+// n = 5000, 64: 11.4 -> 1.46 ms; n = 16000, 4: 3.07 -> 2.6 ms.
 #include <algorithm>
 #include <mutex>
 
@@ -28,8 +27,15 @@ namespace {
 
 constexpr int kSB = 64;           // solve block
 constexpr int kSolveThreads = 256;
-constexpr int kMaxRhsChunk = 8;   // right-hand sides per pass
-constexpr int kAhead = 4;         // pull sweep: factor blocks prefetched into L2 ahead of the fold
+constexpr int kMaxRhsChunk = 8;   // right-hand sides of a group
+// Groups per launch.  A block step's latency does not depend on how many
+// groups run beside it, and the folds' work is shared by all CTAs either way
+// (ms per solve with 1 / 2 / 4 / 8 / 16 groups at most: n = 5000, 64
+// right-hand sides: 6.87 / 3.61 / 2.12 / 1.49 / 1.49; n = 16000, 256: 100 / 63 /
+// 49 / 44 / 43; a sweep that reads the factor once for all of them: 11.4 and
+// 162).
+constexpr int kMaxGroups = 16;
+constexpr int kAhead = 4;         // factor blocks prefetched into L2 ahead of the fold
 
 __global__ void gather_kernel(int n, int nrhs, const double* b, long long ldb, const int* perm,
                               double* y) {
@@ -87,37 +93,13 @@ struct SweepArgs {
   int* status;     // nonzero: a wait ran out; every CTA returns
   int mark;
   unsigned long long timeout_ns;
+  int group_ctas;  // CTAs that share a group of kMaxRhsChunk right-hand sides
 };
 
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-// Waits (thread 0, bounded) until block k is solved; all threads learn
-// whether to go on.
-__device__ bool wait_block(const SweepArgs& A, int k, int* s_ok) {
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    const unsigned long long t0 = globaltimer_ns();
-    for (unsigned it = 1; ld_acquire_s32(A.flags + k) != A.mark; ++it) {
-      if ((it & 31u) == 0) {
-        if (ld_relaxed_s32(A.status) != 0) {
-          ok = 0;
-          break;
-        }
-        if (globaltimer_ns() - t0 > A.timeout_ns) {
-          atomicCAS(A.status, 0, BBK_ERR_TIMEOUT);
-          ok = 0;
-          break;
-        }
-      }
-    }
-    *s_ok = ok;
-  }
-  __syncthreads();
-  return *s_ok != 0;
 }
 
 __device__ __forceinline__ void cp_async_8z(double* smem_dst, const double* gsrc, bool valid) {
@@ -127,165 +109,19 @@ __device__ __forceinline__ void cp_async_8z(double* smem_dst, const double* gsrc
 }
 
 constexpr int kTriPitch = kSB + 1;
-constexpr size_t kSweepSmem = (kSB * kTriPitch + 4 * kMaxRhsChunk * kSB + kMaxRhsChunk * kSB) * sizeof(double);
+constexpr int kInvTmp = 2 * 16 * 17;  // scratch of invert_unit_triangle, doubles
+static_assert(kInvTmp <= 4 * kMaxRhsChunk * kSB, "it fits the partial sums' space");
+constexpr size_t kSweepSmem = (2 * kSB * kTriPitch + 4 * kMaxRhsChunk * kSB + kMaxRhsChunk * kSB) * sizeof(double);
 
-template <bool kForward>
-__global__ void __launch_bounds__(kSolveThreads) psweep_kernel(SweepArgs A) {
-  extern __shared__ double psm[];
-  double* tri = psm;                               // [kSB][kTriPitch]: F(k0+r, k0+c), r < c
-  double (*red)[kMaxRhsChunk][kSB] =
-      reinterpret_cast<double (*)[kMaxRhsChunk][kSB]>(psm + kSB * kTriPitch);  // 4 quarters
-  double (*zs)[kSB] = reinterpret_cast<double (*)[kSB]>(psm + kSB * kTriPitch + 4 * kMaxRhsChunk * kSB);
-  __shared__ int pts[kSB];
-  __shared__ int s_ok;
-  const int n = A.n, nrhs = A.nrhs;
-  const long long ldf = A.ldf;
-  const int nblk = (n + kSB - 1) / kSB;
-  const int G = gridDim.x, c = blockIdx.x;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int row = t & (kSB - 1), quarter = t >> 6;  // 64 rows x 4 quarters of the k range
-  const int dir = kForward ? 1 : -1;
-  // this CTA's blocks in wavefront order: first .. last, stride G
-  const int my_first = kForward ? c : (nblk - 1) - ((nblk - 1 - c) % G);
-  if (kForward ? my_first >= nblk : my_first < 0) return;
-  const int my_last = kForward ? c + ((nblk - 1 - c) / G) * G : c;
-  // the diagonal triangle of an own block, streamed into shared memory ahead of time
-  auto prefetch_tri = [&](int b) {
-    const int b0 = b * kSB, bsz = min(n, b0 + kSB) - b0;
-    for (int idx = t; idx < kSB * kSB; idx += kSolveThreads) {
-      const int r = idx / kSB, cc = idx % kSB;
-      const bool ok = r < cc && cc < bsz;
-      cp_async_8z(&tri[r * kTriPitch + cc], ok ? A.f + static_cast<long long>(b0 + r) * ldf + b0 + cc : A.f, ok);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // factor entries that fold block k into own block b (this thread's 16)
-  auto load_fold = [&](int k, int b, double (&l)[kSB / 4]) {
-    const int k0 = k * kSB, bs = min(n, k0 + kSB) - k0;
-    const int i = b * kSB + row;
-    const int pt_edge = kForward ? A.pt[k0 + bs - 1] : (k0 > 0 ? A.pt[k0 - 1] : 1);
-#pragma unroll
-    for (int u = 0; u < kSB / 4; ++u) {
-      const int kk = quarter * (kSB / 4) + u;
-      const int kg = k0 + kk;
-      bool ok = i < n && kk < bs;
-      double v = 0.0;
-      if (kForward) {
-        // L(i, kg) = F(kg, i); the (kg+1, kg) entry of a 2x2 is zero
-        ok = ok && !(i == kg + 1 && kk == bs - 1 && pt_edge == 2);
-        if (ok) v = A.f[static_cast<long long>(kg) * ldf + i];
-      } else {
-        // L(kg, i) = F(i, kg); the (i+1, i) entry of a 2x2 is zero
-        ok = ok && !(kg == i + 1 && kk == 0 && pt_edge == 2);
-        if (ok) v = A.f[static_cast<long long>(i) * ldf + kg];
-      }
-      l[u] = v;
-    }
-  };
-  prefetch_tri(my_first);
-  for (int step = 0; step < nblk; ++step) {
-    const int k = kForward ? step : nblk - 1 - step;
-    if (kForward ? k > my_last : k < my_last) break;
-    const int k0 = k * kSB, k1 = min(n, k0 + kSB), bs = k1 - k0;
-    const bool mine = k % G == c;
-    // the nearest own block after k receives k's contribution first (critical path)
-    // (the first b beyond k in wavefront order with b % G == c)
-    const int gap = kForward ? (((c - k) % G) + G) % G : (((k - c) % G) + G) % G;
-    const int near = mine ? k + dir * G : k + dir * gap;
-    const bool has_near = kForward ? near <= my_last : near >= my_last;
-    double lnear[kSB / 4];
-    if (has_near) load_fold(k, near, lnear);
-    if (mine) {
-      // ---- own block: every earlier block's contribution is in; solve the triangle
-      for (int r = t; r < kSB; r += kSolveThreads) pts[r] = r < bs ? A.pt[k0 + r] : 1;
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      for (int rc = warp; rc < nrhs; rc += kSolveThreads / 32) {
-        double* yc = A.y + static_cast<long long>(rc) * n;
-        double v0 = lane < bs ? yc[k0 + lane] : 0.0;
-        double v1 = lane + 32 < bs ? yc[k0 + lane + 32] : 0.0;
-        if (kForward) {
-          for (int kk = 0; kk < bs; ++kk) {
-            const double yk = __shfl_sync(0xffffffffu, kk < 32 ? v0 : v1, kk & 31);
-            const bool skip_next = pts[kk] == 2;
-            const int i0 = lane, i1 = lane + 32;
-            if (i0 > kk && i0 < bs && !(skip_next && i0 == kk + 1)) v0 -= tri[kk * kTriPitch + i0] * yk;
-            if (i1 > kk && i1 < bs && !(skip_next && i1 == kk + 1)) v1 -= tri[kk * kTriPitch + i1] * yk;
-          }
-        } else {
-          for (int kk = bs - 1; kk >= 0; --kk) {
-            const double yk = __shfl_sync(0xffffffffu, kk < 32 ? v0 : v1, kk & 31);
-            const int i0 = lane, i1 = lane + 32;
-            // L(kk, i) = F(i, kk) for i < kk, except i == kk-1 opening a 2x2
-            if (i0 < kk && !(i0 == kk - 1 && pts[i0] == 2)) v0 -= tri[i0 * kTriPitch + kk] * yk;
-            if (i1 < kk && !(i1 == kk - 1 && pts[i1] == 2)) v1 -= tri[i1 * kTriPitch + kk] * yk;
-          }
-        }
-        if (lane < bs) yc[k0 + lane] = v0;
-        if (lane + 32 < bs) yc[k0 + lane + 32] = v1;
-      }
-      __syncthreads();
-      if (t == 0) {
-        fence_acq_rel_gpu();
-        asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(A.flags + k), "r"(A.mark) : "memory");
-      }
-      if (has_near) prefetch_tri(near);  // the triangle buffer is free again
-    } else {
-      if (!wait_block(A, k, &s_ok)) return;
-    }
-    // ---- fold block k into this CTA's later blocks
-    for (int c0 = 0; c0 < nrhs; c0 += kMaxRhsChunk) {
-      const int nc = min(kMaxRhsChunk, nrhs - c0);
-      __syncthreads();
-      for (int idx = t; idx < nc * kSB; idx += kSolveThreads) {
-        const int cc = idx / kSB, r = idx % kSB;
-        zs[cc][r] = r < bs ? __ldcg(A.y + static_cast<long long>(c0 + cc) * n + k0 + r) : 0.0;
-      }
-      __syncthreads();
-      for (int b = near; has_near && (kForward ? b <= my_last : b >= my_last); b += dir * G) {
-        double lo[kSB / 4];
-        if (b == near) {
-#pragma unroll
-          for (int u = 0; u < kSB / 4; ++u) lo[u] = lnear[u];
-        } else {
-          load_fold(k, b, lo);
-        }
-        const int b0 = b * kSB;
-        double acc[kMaxRhsChunk];
-#pragma unroll
-        for (int cc = 0; cc < kMaxRhsChunk; ++cc) acc[cc] = 0.0;
-#pragma unroll
-        for (int u = 0; u < kSB / 4; ++u)
-#pragma unroll
-          for (int cc = 0; cc < kMaxRhsChunk; ++cc)
-            if (cc < nc) acc[cc] += lo[u] * zs[cc][quarter * (kSB / 4) + u];
-#pragma unroll
-        for (int cc = 0; cc < kMaxRhsChunk; ++cc)
-          if (cc < nc) red[quarter][cc][row] = acc[cc];
-        __syncthreads();
-        for (int idx = t; idx < nc * kSB; idx += kSolveThreads) {
-          const int cc = idx / kSB, r = idx % kSB;
-          const int ii = b0 + r;
-          if (ii < n) {
-            const double s4 = (red[0][cc][r] + red[1][cc][r]) + (red[2][cc][r] + red[3][cc][r]);
-            A.y[static_cast<long long>(c0 + cc) * n + ii] -= s4;
-          }
-        }
-        __syncthreads();
-      }
-    }
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Pull sweep (at most kMaxRhsChunk right-hand sides per launch).  CTA c owns
-// blocks c, c+G, ... in sweep order and handles one at a time: it folds in
-// the contribution of every earlier block (in sweep order) as soon as that
-// block is solved, then solves the block's own triangle and raises its
-// flag.  Contributions of blocks solved long ago stream in while the blocks
-// just before this one are still being solved elsewhere, so the critical
-// path per block is one flag, one load of the newest solved block, its fold,
-// the reduction and the triangle.
+// One sweep for up to kMaxGroups groups of kMaxRhsChunk right-hand sides, each
+// with CTAs and flags of its own.  CTA c of a group owns blocks c, c+G, ... in
+// sweep order and handles one at a time: it inverts the triangle's two 32 x 32
+// diagonal blocks, folds in the contribution of every earlier block (in sweep
+// order) as soon as that block is solved, then solves the block's own triangle
+// by products with them and raises its flag.  Contributions of blocks solved
+// long ago stream in while the blocks just before this one are still being
+// solved elsewhere, so the critical path per block is one flag, one load of
+// the newest solved block, its fold, the reduction and the triangle.
 //   forward: thread (row, quarter) accumulates L(i, kg) y(kg) over its
 //     quarter of each earlier block (warp loads of F rows are contiguous in
 //     i); the four quarters are added at the end.
@@ -295,8 +131,8 @@ __global__ void __launch_bounds__(kSolveThreads) psweep_kernel(SweepArgs A) {
 // Each warp learns which blocks are solved on its own (one relaxed scan of
 // up to 32 flags, one acquire load of the newest set one, or a bounded wait
 // on the next), so no CTA barrier is taken per block.
-// The triangle is staged so that step kk of the substitution reads row kk
-// of the staged array in both directions (backward: transposed).
+// Substitution through the triangle, one right-hand side per warp, took 2.7
+// of 5.5 us per block; the inverses are ready before the block's turn.
 __device__ __forceinline__ int ld_relaxed_flag(const int* p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -342,18 +178,149 @@ __device__ int warp_wait_solved(const SweepArgs& A, int k, int k_end, int fail) 
   return top;
 }
 
+// inv <- the inverses of the two 32 x 32 diagonal blocks of the unit lower
+// triangle in tri (64 x 64; both by columns: entry (i, k) at [k * kTriPitch
+// + i], entries not below the diagonal zero in tri).  Their 16 x 16 diagonal
+// blocks by substitution, one column per thread, then the blocks below by
+// X21 = -X22 (L21 X11).  Only terms of the triangles enter (an infinity
+// times a zero beside them would not be a zero).  tmp: kInvTmp doubles.
+// Ends with a CTA barrier.
+// (The inverse of the whole triangle left residuals 6 to 15 % larger than
+// substitution does, n = 1000 and 2000; these leave the same.)
+__device__ void invert_unit_triangle(const double* tri, double* inv, double* tmp) {
+  constexpr int P = kTriPitch;
+  const int t = threadIdx.x;
+  for (int idx = t; idx < kSB * P; idx += kSolveThreads) inv[idx] = 0.0;
+  __syncthreads();
+  if (t < kSB) {
+    const int base = t & ~15, j = t & 15;
+    double x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < i; ++k) {
+        const double l = k >= j ? tri[(base + k) * P + base + i] : 0.0;
+        acc = __fma_rn(l, x[k], acc);
+      }
+      x[i] = i == j ? 1.0 : i < j ? 0.0 : -acc;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) inv[(base + j) * P + base + i] = x[i];
+  }
+  __syncthreads();
+  {
+    const int i = t & 15, c = t >> 4;
+    for (int b = 0; b < kSB; b += 32) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double l = k >= c ? tri[(b + k) * P + b + 16 + i] : 0.0;
+        acc = __fma_rn(l, inv[(b + c) * P + b + k], acc);
+      }
+      tmp[(b / 32) * 16 * 17 + c * 17 + i] = acc;
+    }
+    __syncthreads();
+    for (int b = 0; b < kSB; b += 32) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double v = k <= i ? tmp[(b / 32) * 16 * 17 + c * 17 + k] : 0.0;
+        acc = __fma_rn(inv[(b + 16 + k) * P + b + 16 + i], v, acc);
+      }
+      inv[(b + c) * P + b + 16 + i] = -acc;
+    }
+  }
+  __syncthreads();
+}
+
+// The block's triangle, by halves h (backward: the transpose, the second half
+// first): x_h = inv(T_hh) (r_h - T_hg x_g) for the right-hand sides in ys.
+// Each product is 32 x 32: warp w takes the terms 4 w.. of row `lane`, the
+// eight partial sums are added by the thread of (right-hand side, row), which
+// returns its entries lane and lane + 32 of the solution.
+template <bool kForward, bool kMasked>
+__device__ __forceinline__ void solve_triangle(const double* tri, const double* inv, double* red, double* ys, int nc,
+                                               double& x0, double& x1) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int cc0 = warp;
+  auto product = [&](bool masked, const double* m, int rows, int terms) -> double {
+    double acc[kMaxRhsChunk];
+#pragma unroll
+    for (int cc = 0; cc < kMaxRhsChunk; ++cc) acc[cc] = 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = 4 * warp + u;
+      if (masked && (kForward ? k > lane : k < lane)) continue;
+      const double e = kForward ? m[(terms + k) * kTriPitch + rows + lane] : m[(rows + lane) * kTriPitch + terms + k];
+#pragma unroll
+      for (int cc = 0; cc < kMaxRhsChunk; ++cc)
+        if (cc < nc) acc[cc] = __fma_rn(e, ys[cc * kSB + terms + k], acc[cc]);
+    }
+#pragma unroll
+    for (int cc = 0; cc < kMaxRhsChunk; ++cc)
+      if (cc < nc) red[(warp * kMaxRhsChunk + cc) * 32 + lane] = acc[cc];
+    __syncthreads();
+    double sum = 0.0;
+    if (cc0 < nc) {
+      double v[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v[w] = red[(w * kMaxRhsChunk + cc0) * 32 + lane];
+      sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+    return sum;
+  };
+  constexpr int g = kForward ? 0 : 32, h = 32 - g;
+  double* yo = ys + cc0 * kSB;
+  const double xg = product(kMasked, inv, g, g);
+  __syncthreads();  // every term of r_g is read, and every partial sum
+  if (cc0 < nc) yo[g + lane] = xg;
+  __syncthreads();
+  const double th = product(false, tri, h, g);
+  __syncthreads();
+  if (cc0 < nc) yo[h + lane] -= th;
+  __syncthreads();
+  const double xh = product(kMasked, inv, h, h);
+  x0 = kForward ? xg : xh;
+  x1 = kForward ? xh : xg;
+}
+
+// The same from the right-hand sides r0, r1, terms outside the triangle left
+// out; the solution in ys.  (Out of line: it hardly ever runs.)
 template <bool kForward>
-__global__ void __launch_bounds__(kSolveThreads, 1) psweep_pull_kernel(SweepArgs A) {
+__device__ __noinline__ void solve_triangle_masked(const double* tri, const double* inv, double* red, double* ys,
+                                                   int nc, double r0, double r1) {
+  const int lane = threadIdx.x & 31, cc0 = threadIdx.x >> 5;
+  if (cc0 < nc) {
+    ys[cc0 * kSB + lane] = r0;
+    ys[cc0 * kSB + 32 + lane] = r1;
+  }
+  __syncthreads();
+  double x0, x1;
+  solve_triangle<kForward, true>(tri, inv, red, ys, nc, x0, x1);
+  __syncthreads();
+  if (cc0 < nc) {
+    ys[cc0 * kSB + lane] = x0;
+    ys[cc0 * kSB + 32 + lane] = x1;
+  }
+}
+
+template <bool kForward>
+__global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
   extern __shared__ double psm[];
-  double* tri = psm;                            // [kSB][kTriPitch], row kk = step kk's operands
-  double* red = psm + kSB * kTriPitch;          // [4][kMaxRhsChunk][kSB] partial sums
+  double* tri = psm;                            // [kSB][kTriPitch]: the block's triangle, by columns
+  double* inv = tri + kSB * kTriPitch;          // its inverse
+  double* red = inv + kSB * kTriPitch;          // [4][kMaxRhsChunk][kSB] partial sums
   double* ys = red + 4 * kMaxRhsChunk * kSB;    // [kMaxRhsChunk][kSB]: the block being solved
-  __shared__ int pts[kSB];
   __shared__ int s_fail;
-  const int n = A.n, nc = A.nrhs;
+  const int n = A.n;
   const long long ldf = A.ldf;
   const int nblk = (n + kSB - 1) / kSB;
-  const int G = gridDim.x, c = blockIdx.x;
+  // this CTA's group of right-hand sides and its place in it
+  const int G = A.group_ctas, c = blockIdx.x % G, group = blockIdx.x / G;
+  const int nc = min(kMaxRhsChunk, A.nrhs - group * kMaxRhsChunk);
+  A.y += static_cast<long long>(group) * kMaxRhsChunk * n;
+  A.flags += static_cast<long long>(group) * nblk;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int dir = kForward ? 1 : -1;
   const int my_first = kForward ? c : (nblk - 1) - ((nblk - 1 - c) % G);
@@ -364,10 +331,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_pull_kernel(SweepArgs
   auto stage_tri = [&](int b) {
     const int b0 = b * kSB, bsz = min(n, b0 + kSB) - b0;
     for (int idx = t; idx < kSB * kSB; idx += kSolveThreads) {
-      const int r = idx / kSB, cc = idx % kSB;  // F(b0 + r, b0 + cc), r < cc
-      const bool ok = r < cc && cc < bsz;
-      double* dst = kForward ? &tri[r * kTriPitch + cc] : &tri[cc * kTriPitch + r];
-      cp_async_8z(dst, ok ? A.f + static_cast<long long>(b0 + r) * ldf + b0 + cc : A.f, ok);
+      const int r = idx / kSB, cc = idx % kSB;
+      // L(cc, r) = F(b0 + r, b0 + cc), r < cc, except the entry of a 2x2
+      const bool ok = r < cc && cc < bsz && !(cc == r + 1 && A.pt[b0 + r] == 2);
+      cp_async_8z(&tri[r * kTriPitch + cc], ok ? A.f + static_cast<long long>(b0 + r) * ldf + b0 + cc : A.f, ok);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -377,7 +344,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_pull_kernel(SweepArgs
   stage_tri(my_first);
   for (int b = my_first; kForward ? b <= my_last : b >= my_last; b += dir * G) {
     const int b0 = b * kSB, bsz = min(n, b0 + kSB) - b0;
-    for (int r = t; r < kSB; r += kSolveThreads) pts[r] = r < bsz ? A.pt[b0 + r] : 1;
+    // the triangle's inverse, while earlier blocks are still being solved
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    invert_unit_triangle(tri, inv, red);
     // this block's right-hand sides, for the threads that finish them
     double yin[2];
 #pragma unroll
@@ -551,36 +521,25 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_pull_kernel(SweepArgs
         ys[cc * kSB + r] = any ? yin[h] - sum : yin[h];
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // ---- the block's triangle: one warp per right-hand side
-    for (int rc = warp; rc < nc; rc += kSolveThreads / 32) {
-      double* yb = ys + rc * kSB;
-      double v0 = lane < bsz ? yb[lane] : 0.0;
-      double v1 = lane + 32 < bsz ? yb[lane + 32] : 0.0;
-      const int i0 = lane, i1 = lane + 32;
-      // (the backward loop is unrolled over the block so the staged operands
-      // load ahead of the chain; steps past a short last block change
-      // nothing.  Unrolling the forward loop made it slower.)
-      if (kForward) {
-        for (int kk = 0; kk < bsz; ++kk) {
-          const double yk = __shfl_sync(0xffffffffu, kk < 32 ? v0 : v1, kk & 31);
-          const bool skip_next = pts[kk] == 2;
-          if (i0 > kk && i0 < bsz && !(skip_next && i0 == kk + 1)) v0 -= tri[kk * kTriPitch + i0] * yk;
-          if (i1 > kk && i1 < bsz && !(skip_next && i1 == kk + 1)) v1 -= tri[kk * kTriPitch + i1] * yk;
-        }
-      } else {        const bool open0 = pts[i0] == 2, open1 = pts[i1] == 2;
-#pragma unroll
-        for (int kk = kSB - 1; kk >= 0; --kk) {
-          const double yk = __shfl_sync(0xffffffffu, kk < 32 ? v0 : v1, kk & 31);
-          // L(kk, i) = F(i, kk) for i < kk < bsz, except i == kk-1 opening a 2x2
-          if (kk < bsz && i0 < kk && !(i0 == kk - 1 && open0)) v0 -= tri[kk * kTriPitch + i0] * yk;
-          if (kk < bsz && i1 < kk && !(i1 == kk - 1 && open1)) v1 -= tri[kk * kTriPitch + i1] * yk;
-        }
+    // ---- the block's triangle.  The zeros beside a diagonal block's triangle
+    // are harmless while everything is finite, and what is not shows in the
+    // result; then once more with the triangle's terms alone.
+    const int cc0 = t >> 5;  // this thread's right-hand side
+    double* yc = A.y + static_cast<long long>(cc0) * n + b0;
+    const double r0 = cc0 < nc ? ys[cc0 * kSB + lane] : 0.0, r1 = cc0 < nc ? ys[cc0 * kSB + 32 + lane] : 0.0;
+    double x0, x1;
+    solve_triangle<kForward, false>(tri, inv, red, ys, nc, x0, x1);
+    if (cc0 < nc) {
+      if (lane < bsz) yc[lane] = x0;
+      if (lane + 32 < bsz) yc[lane + 32] = x1;
+    }
+    if (__syncthreads_or(!(isfinite(x0) && isfinite(x1)))) {
+      solve_triangle_masked<kForward>(tri, inv, red, ys, nc, r0, r1);
+      if (cc0 < nc) {
+        if (lane < bsz) yc[lane] = ys[cc0 * kSB + lane];
+        if (lane + 32 < bsz) yc[lane + 32] = ys[cc0 * kSB + 32 + lane];
       }
-      double* yc = A.y + static_cast<long long>(rc) * n;
-      if (lane < bsz) yc[b0 + lane] = v0;
-      if (lane + 32 < bsz) yc[b0 + lane + 32] = v1;
     }
     __syncthreads();
     if (t == 0) {
@@ -667,10 +626,6 @@ __global__ void extract_ld_kernel(int n, const double* f, long long ldf, const i
 
 constexpr int kMaxAttrDevices = 64;
 std::once_flag g_sweep_attr[kMaxAttrDevices];
-// right-hand sides up to which the pull sweep is used (in launches of
-// kMaxRhsChunk); more go through the streaming sweep, which reads the
-// factor once for all of them
-constexpr int kPullMaxRhs = 4 * kMaxRhsChunk;
 
 int grid_for(long long work, int threads) {
   const long long g = (work + threads - 1) / threads;
@@ -682,8 +637,7 @@ int grid_for(long long work, int threads) {
 size_t solve_work_doubles(int n, int nrhs) { return 2 * static_cast<size_t>(n) * nrhs; }
 
 int* solve_status_word(double* work, int n, int nrhs) {
-  const int nblk = (n + kSB - 1) / kSB;
-  return reinterpret_cast<int*>(work + static_cast<long long>(n) * nrhs) + nblk;
+  return reinterpret_cast<int*>(work + static_cast<long long>(n) * nrhs);
 }
 
 int solve_status(double* work, int n, int nrhs, cudaStream_t s) {
@@ -695,21 +649,23 @@ int solve_status(double* work, int n, int nrhs, cudaStream_t s) {
 }
 
 // work: 2 n nrhs doubles: the right-hand sides being solved in place, then
-// the block flags and the status word.
+// the status word and the block flags (one set per group of right-hand sides).
 int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const int* pivot_types,
                   int nrhs, double* b, long long ldb, double* work, cudaStream_t s) {
   double* y = work;
   const long long total = static_cast<long long>(n) * nrhs;
   const int nblk = (n + kSB - 1) / kSB;
-  int* flags = reinterpret_cast<int*>(work + total);
   int* status = solve_status_word(work, n, nrhs);
-  reset_flags_kernel<<<std::max(1, std::min(64, (nblk + 256) / 256)), 256, 0, s>>>(flags, nblk + 1);
+  int* flags = status + 1;
+  const int ngroups = (nrhs + kMaxRhsChunk - 1) / kMaxRhsChunk;
+  const int nflags = 1 + ngroups * nblk;
+  reset_flags_kernel<<<std::max(1, std::min(64, (nflags + 255) / 256)), 256, 0, s>>>(status, nflags);
   BBK_CUDA_TRY(cudaGetLastError());
   count_launch();
   gather_kernel<<<grid_for(total, 256), 256, 0, s>>>(n, nrhs, b, ldb, perm, y);
   BBK_CUDA_TRY(cudaGetLastError());
   count_launch();
-  SweepArgs A{n, nrhs, f, ldf, pivot_types, y, flags, status, 1, wait_timeout_ns()};
+  SweepArgs A{n, nrhs, f, ldf, pivot_types, y, flags, status, 1, wait_timeout_ns(), 1};
   // both sweeps need more than the default 48 KB of dynamic shared memory;
   // the attributes are set per device, each under its own once-flag
   // (callers may be on several host threads)
@@ -718,38 +674,31 @@ int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const 
   if (dev < 0 || dev >= kMaxAttrDevices) return set_error(BBK_ERR_NO_DEVICE, "device %d out of range", dev);
   cudaError_t attr_err = cudaSuccess;
   std::call_once(g_sweep_attr[dev], [&] {
-    const void* fns[4] = {reinterpret_cast<const void*>(psweep_kernel<true>),
-                          reinterpret_cast<const void*>(psweep_kernel<false>),
-                          reinterpret_cast<const void*>(psweep_pull_kernel<true>),
-                          reinterpret_cast<const void*>(psweep_pull_kernel<false>)};
-    for (int i = 0; i < 4 && attr_err == cudaSuccess; ++i)
+    const void* fns[2] = {reinterpret_cast<const void*>(psweep_kernel<true>),
+                          reinterpret_cast<const void*>(psweep_kernel<false>)};
+    for (int i = 0; i < 2 && attr_err == cudaSuccess; ++i)
       attr_err = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kSweepSmem));
   });
   BBK_CUDA_TRY(attr_err);
-  const int grid = std::max(1, std::min(nblk, device_sm_count()));
-  auto sweep = [&](const void* fn, SweepArgs& args) -> int {
-    void* kargs[] = {&args};
-    BBK_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolveThreads), kargs, kSweepSmem, s));
-    count_launch();
-    return BBK_OK;
-  };
-  const bool pull = nrhs <= kPullMaxRhs;
+  const int sms = device_sm_count();
   // every sweep launch waits for its own flag value
   int mark = 0;
   auto sweeps = [&](bool forward) -> int {
-    const void* fn = pull ? (forward ? reinterpret_cast<const void*>(psweep_pull_kernel<true>)
-                                     : reinterpret_cast<const void*>(psweep_pull_kernel<false>))
-                          : (forward ? reinterpret_cast<const void*>(psweep_kernel<true>)
-                                     : reinterpret_cast<const void*>(psweep_kernel<false>));
-    const int chunk = pull ? kMaxRhsChunk : nrhs;
+    const void* fn = forward ? reinterpret_cast<const void*>(psweep_kernel<true>)
+                             : reinterpret_cast<const void*>(psweep_kernel<false>);
+    constexpr int chunk = kMaxGroups * kMaxRhsChunk;
     for (int c0 = 0; c0 < nrhs; c0 += chunk) {
       SweepArgs a = A;
       a.y = y + static_cast<long long>(c0) * n;
       a.nrhs = std::min(chunk, nrhs - c0);
       a.mark = ++mark;
-      const int rc = sweep(fn, a);
-      if (rc) return rc;
+      const int groups = (a.nrhs + kMaxRhsChunk - 1) / kMaxRhsChunk;
+      a.group_ctas = std::max(1, std::min(nblk, sms / groups));
+      void* kargs[] = {&a};
+      BBK_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(groups * a.group_ctas), dim3(kSolveThreads), kargs,
+                                               kSweepSmem, s));
+      count_launch();
     }
     return BBK_OK;
   };
