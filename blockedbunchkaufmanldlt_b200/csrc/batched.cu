@@ -17,6 +17,17 @@
 // is updated from the shared-memory W and U with register-tiled FMAs.  A
 // itself stays in global memory (L2-resident while the CTA works on it).
 //
+// One CTA per SM left three quarters of the issue slots empty: a pivot step is
+// a chain of barriers and short latencies.  Two CTAs share an SM now.  Where
+// W and U together take more than half of its shared memory (FP64, order 256
+// with block 32 and up), U is not kept (see the lean layout).  Launches with
+// one, two or four slots per thread drop the idle iterations, and tiles
+// inside the triangle and row copies go without a bounds check or a division
+// per element.  4096 KKT matrices of order 16..512: 28.1 -> 17.9 ms; 1184 of
+// order 512 / 256 / 128 / 64: 22.7 -> 16.3, 6.1 -> 3.6, 2.7 -> 1.5, 1.3 -> 0.8 ms
+// (copies included).  W and U both kept in narrower panels (block 8 at order
+// 512) took 24.3 ms at order 512: the trailing matrix is read once per panel.
+//
 // Arithmetic modes: FP64_ORDERED reproduces the reference bit for bit
 // (ordered dot products and trailing sums, every product and sum rounded
 // separately); FP64 reassociates them into FMA chains; FP32 runs the
@@ -34,11 +45,11 @@ namespace {
 
 constexpr int kBT = 256;              // threads per CTA
 constexpr int kBWarps = kBT / 32;
-constexpr int kBC = (BBK_BATCH_MAX_N + kBT - 1) / kBT;  // slots per thread
 constexpr int kMaxB = 64;             // largest block size
 constexpr int kCap = 2 * kMaxB + 4;   // moved indices per panel
 constexpr int kWU = kMaxB + 2;        // a panel has at most b + 1 pivot rows
 constexpr size_t kBatchSmem = 220 * 1024;
+constexpr size_t kHalfSmem = 112 * 1024;  // two CTAs per SM
 constexpr int kSolveBlk = 32;
 
 struct BatchItemDev {
@@ -62,12 +73,13 @@ struct BatchArgs {
   double* scratch;        // per CTA: gbuf (kCap x max_n), gbuf2 (max_n x kCap), vectors
   long long scratch_stride;
   int max_n;
+  int lean;               // items that take more than half of an SM's shared memory in the lean layout
 };
 
 // Shared-memory carve-up for one item.
 struct Smem {
   double* wsm;   // (b+2) x nw: staged panel rows -> workspace rows, by slot
-  double* usm;   // n x ldu: U by slot
+  double* usm;   // (b+2) x nw: U by slot
   double* wcs;   // n: candidate column by slot (also the solve vector)
   double* dlog;  // 2 (b+2)
   double* red_v; // 2 x kBWarps (alternating reductions)
@@ -78,35 +90,93 @@ struct Smem {
   int* red_i;    // 2 x kBWarps
   int* red_s;    // 2 x kBWarps
   int* misc;     // 8
-  double* tile;  // kSolveBlk x (kSolveBlk + 1): a diagonal block of the factor (solve)
+  double* tile;  // kSolveBlk x (kSolveBlk + 1): a diagonal block of the factor (solve; in the lean
+                 // layout over wsm)
+  double* ua;    // lean layout, b+2 each: how U's row q follows from W (see u_value), and the
+  double* ub;    // coefficient column of a step
+  double* coef;
+  int* upk;
   int* tpt;      // kSolveBlk: that block's pivot types
-  int ldu;
   int nw;
 };
 
-// U and W leading dimensions = 4 (mod 16) doubles: the tensor-core fragment
+// U and W leading dimension = 4 (mod 16) doubles: the tensor-core fragment
 // loads of the trailing update are then free of bank conflicts.
-__host__ __device__ inline int batch_ldu(int b) { return (b + 2 + 11) / 16 * 16 + 4; }
 __host__ __device__ inline int batch_nw(int n) { return (n + 11) / 16 * 16 + 4; }
 
-__host__ __device__ inline size_t batch_smem_bytes(int n, int b) {
-  const size_t nd = static_cast<size_t>(b + 2) * batch_nw(n) + static_cast<size_t>(n) * batch_ldu(b) + n +
+// Bounds the block size of an order (with U by columns, as it was laid out
+// when the bound was set: a plan's block sizes do not depend on the layout).
+inline size_t batch_block_bytes(int n, int b) {
+  const size_t ldu = (b + 2 + 11) / 16 * 16 + 4;
+  const size_t nd = static_cast<size_t>(b + 2) * batch_nw(n) + static_cast<size_t>(n) * ldu + n +
                     2 * static_cast<size_t>(b + 2) + 2 * kBWarps + kSolveBlk * (kSolveBlk + 1);
   const size_t ni = static_cast<size_t>(b + 2) + 2 * static_cast<size_t>(n) + kCap + 4 * kBWarps + 8 + kSolveBlk;
   return nd * sizeof(double) + ni * sizeof(int);
 }
 
+__host__ __device__ inline size_t batch_smem_bytes(int n, int b) {
+  const size_t nd = 2 * static_cast<size_t>(b + 2) * batch_nw(n) + n +
+                    2 * static_cast<size_t>(b + 2) + 2 * kBWarps + kSolveBlk * (kSolveBlk + 1);
+  const size_t ni = static_cast<size_t>(b + 2) + 2 * static_cast<size_t>(n) + kCap + 4 * kBWarps + 8 + kSolveBlk;
+  return nd * sizeof(double) + ni * sizeof(int);
+}
+
+// The lean layout: no U.  U's columns are formed from W when a step needs
+// them, and the trailing update reads U's rows where the compact factors have
+// them.  Half the shared memory, so two CTAs share an SM.
+__host__ __device__ inline size_t batch_lean_bytes(int n, int b) {
+  const size_t w = static_cast<size_t>(b + 2) * batch_nw(n);
+  const size_t tile = kSolveBlk * (kSolveBlk + 1);
+  const size_t nd = (w > tile ? w : tile) + n + 5 * static_cast<size_t>(b + 2) + 2 * kBWarps;
+  const size_t ni = 2 * static_cast<size_t>(b + 2) + 2 * static_cast<size_t>(n) + kCap + 4 * kBWarps + 8 + kSolveBlk;
+  return nd * sizeof(double) + ni * sizeof(int);
+}
+
+// The panel width the lean layout holds of a planned block (FP64 only: the
+// pivots do not depend on it).
+__host__ __device__ inline int lean_block(int n, int b) {
+  while (b > 1 && batch_lean_bytes(n, b) > kHalfSmem) --b;
+  return b;
+}
+
+// Shared memory of an item when two CTAs share an SM.
+inline size_t batch_half_bytes(int n, int b) {
+  const size_t full = batch_smem_bytes(n, b);
+  return full <= kHalfSmem ? full : batch_lean_bytes(n, lean_block(n, b));
+}
+
+template <bool kLean>
 __device__ Smem carve(double* base, int n, int b) {
   Smem S;
-  S.ldu = batch_ldu(b);
   S.nw = batch_nw(n);
+  const size_t w = static_cast<size_t>(b + 2) * S.nw;
+  const size_t tile = kSolveBlk * (kSolveBlk + 1);
   S.wsm = base;
-  S.usm = S.wsm + static_cast<size_t>(b + 2) * S.nw;
-  S.wcs = S.usm + static_cast<size_t>(n) * S.ldu;
+  if (kLean) {
+    S.usm = S.wsm;  // (not used; the refinement's scratch)
+    S.tile = S.wsm;
+    S.wcs = S.wsm + (w > tile ? w : tile);
+  } else {
+    S.usm = S.wsm + w;
+    S.wcs = S.usm + w;
+  }
   S.dlog = S.wcs + n;
   S.red_v = S.dlog + 2 * (b + 2);
-  S.tile = S.red_v + 2 * kBWarps;
-  int* ib = reinterpret_cast<int*>(S.tile + kSolveBlk * (kSolveBlk + 1));
+  double* end = S.red_v + 2 * kBWarps;
+  if (kLean) {
+    S.ua = end;
+    S.ub = S.ua + (b + 2);
+    S.coef = S.ub + (b + 2);
+    end = S.coef + (b + 2);
+  } else {
+    S.tile = end;
+    end += tile;
+  }
+  int* ib = reinterpret_cast<int*>(end);
+  if (kLean) {
+    S.upk = ib;
+    ib += b + 2;
+  }
   S.win = ib;
   S.mypos = S.win + (b + 2);
   S.srcmap = S.mypos + n;
@@ -118,12 +188,31 @@ __device__ Smem carve(double* base, int n, int b) {
   return S;
 }
 
-__device__ __forceinline__ void argmax_join3(double& v, int& i, int& s, double v2, int i2, int s2) {
-  if (v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
-    s = s2;
-  }
+// U[q, z] from W, as the scaling phase would have stored it (upk: 1 a 1x1
+// pivot, W / ua; 2 the first, 3 the second row of a 2x2 with its
+// coefficients).
+__device__ __forceinline__ double u_value(const Smem& S, int q, int z) {
+  const int kind = S.upk[q];
+  const double x = S.wsm[q * S.nw + z];
+  if (kind == 1) return div_or_zero(x, S.ua[q]);
+  if (kind == 2) return xadd(xmul(S.ua[q], x), xmul(S.ub[q], S.wsm[(q + 1) * S.nw + z]));
+  return xadd(xmul(S.ua[q], S.wsm[(q - 1) * S.nw + z]), xmul(S.ub[q], x));
+}
+
+// Warp argmax: the values are never negative or NaN, so their bit patterns
+// order like the values and integer reductions find the largest (high word,
+// low word, then the lowest index); every lane gets the result.
+__device__ __forceinline__ void warp_argmax3(double& v, int& i, int& s) {
+  const unsigned long long key = static_cast<unsigned long long>(__double_as_longlong(v));
+  const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+  const bool top = hi == mhi && lo == mlo;
+  const unsigned midx = __reduce_min_sync(0xffffffffu, top ? static_cast<unsigned>(i) : 0xffffffffu);
+  const int who = __ffs(__ballot_sync(0xffffffffu, top && static_cast<unsigned>(i) == midx)) - 1;
+  v = __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(mhi) << 32) | mlo));
+  i = static_cast<int>(midx);
+  s = __shfl_sync(0xffffffffu, s, who);
 }
 
 // CTA argmax (value, index, slot) with the reference's tie rule; every
@@ -132,12 +221,7 @@ __device__ __forceinline__ void argmax_join3(double& v, int& i, int& s, double v
 // only after the barrier of the reduction in between.
 __device__ void block_argmax(const Smem& S, int& parity, double& v, int& i, int& s) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int off = 16; off > 0; off >>= 1) {
-    const double v2 = __shfl_down_sync(0xffffffffu, v, off);
-    const int i2 = __shfl_down_sync(0xffffffffu, i, off);
-    const int s2 = __shfl_down_sync(0xffffffffu, s, off);
-    argmax_join3(v, i, s, v2, i2, s2);
-  }
+  warp_argmax3(v, i, s);
   const int base = parity * kBWarps;
   parity ^= 1;
   if (lane == 0) {
@@ -146,11 +230,28 @@ __device__ void block_argmax(const Smem& S, int& parity, double& v, int& i, int&
     S.red_s[base + warp] = s;
   }
   __syncthreads();
-  v = S.red_v[base];
-  i = S.red_i[base];
-  s = S.red_s[base];
-  for (int k = 1; k < kBWarps; ++k)
-    argmax_join3(v, i, s, S.red_v[base + k], S.red_i[base + k], S.red_s[base + k]);
+  v = lane < kBWarps ? S.red_v[base + lane] : 0.0;
+  i = lane < kBWarps ? S.red_i[base + lane] : INT_MAX;
+  s = lane < kBWarps ? S.red_s[base + lane] : -1;
+  warp_argmax3(v, i, s);
+}
+
+// CTA maximum of values that are never negative or NaN, likewise.
+__device__ double block_max(const Smem& S, int& parity, double v) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto warp_max = [](double x) {
+    const unsigned long long key = static_cast<unsigned long long>(__double_as_longlong(x));
+    const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    return __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(mhi) << 32) | mlo));
+  };
+  v = warp_max(v);
+  const int base = parity * kBWarps;
+  parity ^= 1;
+  if (lane == 0) S.red_v[base + warp] = v;
+  __syncthreads();
+  return warp_max(lane < kBWarps ? S.red_v[base + lane] : 0.0);
 }
 
 __device__ __forceinline__ void cp_async_8(double* smem_dst, const double* gsrc) {
@@ -159,22 +260,32 @@ __device__ __forceinline__ void cp_async_8(double* smem_dst, const double* gsrc)
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// for idx in [0, total): st(idx, ld(idx)), each thread keeping kDepth loads
-// in flight (the loads do not wait on the stores)
+// for r in [0, rows), c in [0, cols): st(r, c, ld(r, c)), a row per warp and a
+// column per lane (no division), kDepth loads in flight per thread (the
+// loads do not wait on the stores)
 template <int kDepth, typename Ld, typename St>
-__device__ __forceinline__ void pipelined_copy(int total, Ld&& ld, St&& st) {
-  for (int base = threadIdx.x; base < total; base += kBT * kDepth) {
-    double v[kDepth];
+__device__ __forceinline__ void copy_rows(int rows, int cols, Ld&& ld, St&& st) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (cols >= 32 * kDepth / 2) {  // wide rows: several columns of one row in flight
+    for (int r = warp; r < rows; r += kBWarps)
+      for (int c0 = lane; c0 < cols; c0 += 32 * kDepth) {
+        double v[kDepth];
 #pragma unroll
-    for (int u = 0; u < kDepth; ++u) {
-      const int idx = base + u * kBT;
-      v[u] = idx < total ? ld(idx) : 0.0;
-    }
+        for (int u = 0; u < kDepth; ++u) v[u] = c0 + 32 * u < cols ? ld(r, c0 + 32 * u) : 0.0;
 #pragma unroll
-    for (int u = 0; u < kDepth; ++u) {
-      const int idx = base + u * kBT;
-      if (idx < total) st(idx, v[u]);
-    }
+        for (int u = 0; u < kDepth; ++u)
+          if (c0 + 32 * u < cols) st(r, c0 + 32 * u, v[u]);
+      }
+  } else {  // narrow ones: one column of several rows
+    for (int c = lane; c < cols; c += 32)
+      for (int r0 = warp; r0 < rows; r0 += kBWarps * kDepth) {
+        double v[kDepth];
+#pragma unroll
+        for (int u = 0; u < kDepth; ++u) v[u] = r0 + kBWarps * u < rows ? ld(r0 + kBWarps * u, c) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kDepth; ++u)
+          if (r0 + kBWarps * u < rows) st(r0 + kBWarps * u, c, v[u]);
+      }
   }
 }
 
@@ -197,15 +308,17 @@ __device__ __forceinline__ void mma_f64_16x8x8(double (&c)[4], const double (&a)
 
 // FP64 tensor cores: each warp owns 32 x 32 tiles of the upper tile
 // triangle (2 x 4 fragments of m16n8k8).
+template <bool kLean>
 __device__ void trailing_dmma(const Smem& S, double* A, int lda, int n, int e, int kb) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tq = lane & 3;
   const int m = n - e;
   const int tiles = (m + 31) / 32;
   const int ntile = tiles * (tiles + 1) / 2;
-  const double* U = S.usm;
+  // lean: U's rows from the compact factors just written
+  const double* U = kLean ? A + static_cast<long long>(e - kb) * lda : S.usm;
   const double* W = S.wsm;
-  const int ldu = S.ldu, nw = S.nw;
+  const int nw = S.nw, nu = kLean ? lda : nw;
   for (int tid = warp; tid < ntile; tid += kBWarps) {
     int J = static_cast<int>((sqrtf(8.0f * tid + 1.0f) - 1.0f) * 0.5f);
     while (J * (J + 1) / 2 > tid) --J;
@@ -213,16 +326,45 @@ __device__ void trailing_dmma(const Smem& S, double* A, int lda, int n, int e, i
     const int I = tid - J * (J + 1) / 2;
     const int i0 = e + 32 * I, j0 = e + 32 * J;
     double acc[2][4][4] = {};
-    for (int ks = 0; ks < kb; ks += 8) {
+    int ks = 0;
+    const bool inside = I < J && j0 + 32 <= n;
+    if (inside) {
+      // no bounds inside the triangle, and whole k steps: plain offsets from
+      // two pointers (with a check per element nine tenths of the kernel's
+      // instructions were addresses and predicates)
+      const double* up = U + static_cast<long long>(tq) * nu + i0 + g;
+      const double* wp = W + tq * nw + j0 + g;
+      for (; ks + 8 <= kb; ks += 8, up += 8 * static_cast<long long>(nu), wp += 8 * nw) {
+        const double *u1 = up + 4 * static_cast<long long>(nu), *w1 = wp + 4 * nw;
+        double af[2][4], bf[4][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          af[mt][0] = up[mt * 16];
+          af[mt][1] = up[mt * 16 + 8];
+          af[mt][2] = u1[mt * 16];
+          af[mt][3] = u1[mt * 16 + 8];
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          bf[nt][0] = wp[nt * 8];
+          bf[nt][1] = w1[nt * 8];
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) mma_f64_16x8x8(acc[mt][nt], af[mt], bf[nt]);
+      }
+    }
+    for (; ks < kb; ks += 8) {
       const int k0 = ks + tq, k1 = ks + tq + 4;
       double af[2][4], bf[4][2];
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
         const int r0 = i0 + mt * 16 + g, r1 = r0 + 8;
-        af[mt][0] = (r0 < n && k0 < kb) ? U[static_cast<size_t>(r0) * ldu + k0] : 0.0;
-        af[mt][1] = (r1 < n && k0 < kb) ? U[static_cast<size_t>(r1) * ldu + k0] : 0.0;
-        af[mt][2] = (r0 < n && k1 < kb) ? U[static_cast<size_t>(r0) * ldu + k1] : 0.0;
-        af[mt][3] = (r1 < n && k1 < kb) ? U[static_cast<size_t>(r1) * ldu + k1] : 0.0;
+        af[mt][0] = (r0 < n && k0 < kb) ? U[static_cast<long long>(k0) * nu + r0] : 0.0;
+        af[mt][1] = (r1 < n && k0 < kb) ? U[static_cast<long long>(k0) * nu + r1] : 0.0;
+        af[mt][2] = (r0 < n && k1 < kb) ? U[static_cast<long long>(k1) * nu + r0] : 0.0;
+        af[mt][3] = (r1 < n && k1 < kb) ? U[static_cast<long long>(k1) * nu + r1] : 0.0;
       }
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
@@ -235,7 +377,48 @@ __device__ void trailing_dmma(const Smem& S, double* A, int lda, int n, int e, i
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) mma_f64_16x8x8(acc[mt][nt], af[mt], bf[nt]);
     }
-    // C -= acc: every load of the tile first, then every store
+    // C -= acc: loads before stores
+    if (inside) {
+      double* cp = A + static_cast<long long>(i0 + g) * lda + j0 + 2 * tq;
+      const bool pairs = ((reinterpret_cast<uintptr_t>(A + e) | (static_cast<uintptr_t>(lda) * sizeof(double))) & 15) == 0;
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        double* c0 = cp + static_cast<long long>(mt * 16) * lda;
+        double* c1 = c0 + 8 * static_cast<long long>(lda);
+        if (pairs) {  // half the cache lines per instruction
+          double2 w0[4], w1[4];
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            w0[nt] = *reinterpret_cast<const double2*>(c0 + nt * 8);
+            w1[nt] = *reinterpret_cast<const double2*>(c1 + nt * 8);
+          }
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            *reinterpret_cast<double2*>(c0 + nt * 8) =
+                make_double2(w0[nt].x - acc[mt][nt][0], w0[nt].y - acc[mt][nt][1]);
+            *reinterpret_cast<double2*>(c1 + nt * 8) =
+                make_double2(w1[nt].x - acc[mt][nt][2], w1[nt].y - acc[mt][nt][3]);
+          }
+          continue;
+        }
+        double v[4][4];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          v[nt][0] = c0[nt * 8];
+          v[nt][1] = c0[nt * 8 + 1];
+          v[nt][2] = c1[nt * 8];
+          v[nt][3] = c1[nt * 8 + 1];
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          c0[nt * 8] = v[nt][0] - acc[mt][nt][0];
+          c0[nt * 8 + 1] = v[nt][1] - acc[mt][nt][1];
+          c1[nt * 8] = v[nt][2] - acc[mt][nt][2];
+          c1[nt * 8 + 1] = v[nt][3] - acc[mt][nt][3];
+        }
+      }
+      continue;
+    }
     double cv[2][4][4];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -297,7 +480,7 @@ __device__ void trailing_simt(const Smem& S, double* A, int lda, int n, int e, i
         float uv[4], wv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          uv[u] = static_cast<float>(S.usm[static_cast<size_t>(ri[u]) * S.ldu + q]);
+          uv[u] = static_cast<float>(S.usm[q * S.nw + ri[u]]);
           wv[u] = static_cast<float>(S.wsm[q * S.nw + cj[u]]);
         }
 #pragma unroll
@@ -319,7 +502,7 @@ __device__ void trailing_simt(const Smem& S, double* A, int lda, int n, int e, i
         double uv[4], wv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          uv[u] = S.usm[static_cast<size_t>(ri[u]) * S.ldu + q];
+          uv[u] = S.usm[q * S.nw + ri[u]];
           wv[u] = S.wsm[q * S.nw + cj[u]];
         }
 #pragma unroll
@@ -339,10 +522,19 @@ __device__ void trailing_simt(const Smem& S, double* A, int lda, int n, int e, i
   }
 }
 
+// One slot's column of U (or W): row q at p[q * pitch].
+struct Column {
+  const double* p;
+  int pitch;
+  __device__ __forceinline__ double operator[](int q) const { return p[q * pitch]; }
+};
+
 // ---------------------------------------------------------------------------
 // Factorization of one matrix by one CTA
 // ---------------------------------------------------------------------------
-template <int kMode>  // BBK_UPDATE_FP64_ORDERED, BBK_UPDATE_FP64 or BBK_UPDATE_FP32
+// kMode: BBK_UPDATE_FP64_ORDERED, BBK_UPDATE_FP64 or BBK_UPDATE_FP32; kC: slots
+// per thread (the batch's largest order / kBT).
+template <int kMode, int kC, bool kLean>
 __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int* perm, int* pt,
                            double* gbuf, double* gbuf2, int* permbuf, double* wutmp) {
   constexpr bool kOrdered = kMode == BBK_UPDATE_FP64_ORDERED;
@@ -362,11 +554,12 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
     // ---- stage the panel rows; identity maps
     for (int m = t; m < nwin; m += kBT) S.win[m] = k0 + m;
     for (int z = k0 + t; z < n; z += kBT) S.mypos[z] = z;
-    for (int idx = t; idx < nwin * (n - k0); idx += kBT) {
-      const int m = idx / (n - k0), z = k0 + idx % (n - k0);
+    for (int m = t >> 5; m < nwin; m += kBWarps) {
       const int x = k0 + m;
-      cp_async_8(&S.wsm[m * nw + z], x <= z ? A + static_cast<long long>(x) * lda + z
-                                           : A + static_cast<long long>(z) * lda + x);
+      const double* row = A + static_cast<long long>(x) * lda;
+      double* dst = S.wsm + m * nw;
+      for (int z = k0 + (t & 31); z < n; z += 32)
+        cp_async_8(dst + z, x <= z ? row + z : A + static_cast<long long>(z) * lda + x);
     }
     cp_async_wait_all();
     if (t == 0) S.misc[0] = 0;
@@ -377,12 +570,16 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
       const int lp = p - k0;
       const int sp = S.win[lp];
       const bool staged = sp - k0 == lp;
-      const double* ucol = S.usm + static_cast<size_t>(sp) * S.ldu;
+      if (kLean) {
+        if (t < lp) S.coef[t] = u_value(S, t, sp);
+        __syncthreads();
+      }
+      const Column ucol = kLean ? Column{S.coef, 1} : Column{S.usm + sp, nw};
       // ---- row update W[p, j] = A[p, j] - sum_q U[q, p] W[q, j]  (:122-182)
       double best = 0.0;
       int best_j = INT_MAX, best_z = -1;
 #pragma unroll
-      for (int k = 0; k < kBC; ++k) {
+      for (int k = 0; k < kC; ++k) {
         const int z = k0 + t + k * kBT;
         if (z < n && S.mypos[z] >= p) {
           const double av = staged ? S.wsm[lp * nw + z] : asym(A, lda, sp, z);
@@ -415,10 +612,14 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
       if (!(fabs(dpp) >= xmul(kAlpha, omega) || omega == 0.0)) {  // :90-92
         cand = true;
         // ---- candidate column W(i, r) = A(i, r) - sum_q U[q, r] W[q, i]  (:184-367)
-        const double* rcol = S.usm + static_cast<size_t>(rs) * S.ldu;
+        if (kLean) {
+          if (t < lp) S.coef[t] = u_value(S, t, rs);
+          __syncthreads();
+        }
+        const Column rcol = kLean ? Column{S.coef, 1} : Column{S.usm + rs, nw};
         double sig = 0.0;
 #pragma unroll
-        for (int k = 0; k < kBC; ++k) {
+        for (int k = 0; k < kC; ++k) {
           const int z = k0 + t + k * kBT;
           if (z < n && S.mypos[z] >= p) {
             const double cv = asym(A, lda, z, rs);
@@ -432,9 +633,7 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
             }
           }
         }
-        int di = 0, ds = 0;
-        block_argmax(S, red_parity, sig, di, ds);
-        const double sigma = sig;
+        const double sigma = block_max(S, red_parity, sig);
         wc_r = S.wcs[rs];
         wc_p = S.wcs[sp];
         if (xsub(xmul(fabs(dpp), sigma), xmul(xmul(kAlpha, omega), omega)) >= 0.0) {  // :369-390
@@ -454,7 +653,7 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
       if (kind == 1) {  // ScaleOneByOnePivot :633-656
         const double d = dpp, den = safe_denominator(d);
 #pragma unroll
-        for (int k = 0; k < kBC; ++k) {
+        for (int k = 0; k < kC; ++k) {
           const int z = k0 + t + k * kBT;
           if (z < n && S.mypos[z] > p) {
             double wv = S.wsm[lp * nw + z];
@@ -462,12 +661,16 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
               wv = wc_p;
               S.wsm[lp * nw + z] = wv;
             }
-            S.usm[static_cast<size_t>(z) * S.ldu + lp] = div_or_zero(wv, den);
+            if (!kLean) S.usm[lp * nw + z] = div_or_zero(wv, den);
           }
         }
         if (t == 0) {
           S.dlog[2 * lp] = d;
           pt[p] = 1;
+          if (kLean) {
+            S.upk[lp] = 1;
+            S.ua[lp] = den;
+          }
         }
         p += 1;
       } else if (kind == -1) {  // SwapOneByOnePivot + ScaleOneByOnePivot
@@ -479,15 +682,19 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
           S.mypos[rs] = p;
           S.dlog[2 * lp] = d;
           pt[p] = 1;
+          if (kLean) {
+            S.upk[lp] = 1;
+            S.ua[lp] = den;
+          }
         }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kBC; ++k) {
+        for (int k = 0; k < kC; ++k) {
           const int z = k0 + t + k * kBT;
           if (z < n && S.mypos[z] > p) {
             const double wv = S.wcs[z];
             S.wsm[lp * nw + z] = wv;
-            S.usm[static_cast<size_t>(z) * S.ldu + lp] = div_or_zero(wv, den);
+            if (!kLean) S.usm[lp * nw + z] = div_or_zero(wv, den);
           }
         }
         p += 1;
@@ -508,16 +715,26 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
           S.dlog[2 * ls] = d22;
           pt[p] = 2;
           pt[p + 1] = -2;
+          if (kLean) {
+            S.upk[lp] = 2;
+            S.ua[lp] = i11;
+            S.ub[lp] = i21;
+            S.upk[ls] = 3;
+            S.ua[ls] = i21;
+            S.ub[ls] = i22;
+          }
         }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kBC; ++k) {
+        for (int k = 0; k < kC; ++k) {
           const int z = k0 + t + k * kBT;
           if (z < n && S.mypos[z] > p + 1) {
             const double xv = S.wsm[lp * nw + z], yv = S.wcs[z];
             S.wsm[ls * nw + z] = yv;
-            S.usm[static_cast<size_t>(z) * S.ldu + lp] = xadd(xmul(i11, xv), xmul(i21, yv));
-            S.usm[static_cast<size_t>(z) * S.ldu + ls] = xadd(xmul(i21, xv), xmul(i22, yv));
+            if (!kLean) {
+              S.usm[lp * nw + z] = xadd(xmul(i11, xv), xmul(i21, yv));
+              S.usm[ls * nw + z] = xadd(xmul(i21, xv), xmul(i22, yv));
+            }
           }
         }
         p += 2;
@@ -537,69 +754,68 @@ __device__ void factor_one(const Smem& S, double* A, int n, int lda, int b, int*
     const int m = n - k0;
     // gather: rows of the moved indices, factored rows at the moved
     // columns, permutation entries, and the moved W columns / U rows
-    pipelined_copy<8>(
-        cnt * m,
-        [&](int idx) {
-          const int ix = idx / m, y = k0 + idx % m;
-          return asym(A, lda, S.srcmap[S.moved[ix]], S.srcmap[y]);
-        },
-        [&](int idx, double v) { gbuf[static_cast<long long>(idx / m) * n + k0 + idx % m] = v; });
-    pipelined_copy<8>(
-        k0 * cnt,
-        [&](int idx) { return A[static_cast<long long>(idx / cnt) * lda + S.srcmap[S.moved[idx % cnt]]]; },
-        [&](int idx, double v) { gbuf2[static_cast<long long>(idx / cnt) * kCap + idx % cnt] = v; });
+    copy_rows<8>(
+        cnt, m, [&](int ix, int c) { return asym(A, lda, S.srcmap[S.moved[ix]], S.srcmap[k0 + c]); },
+        [&](int ix, int c, double v) { gbuf[static_cast<long long>(ix) * n + k0 + c] = v; });
+    copy_rows<8>(
+        k0, cnt, [&](int q, int ix) { return A[static_cast<long long>(q) * lda + S.srcmap[S.moved[ix]]]; },
+        [&](int q, int ix, double v) { gbuf2[static_cast<long long>(q) * kCap + ix] = v; });
     for (int ix = t; ix < cnt; ix += kBT) permbuf[ix] = perm[S.srcmap[S.moved[ix]]];
-    for (int idx = t; idx < cnt * kb; idx += kBT) {
-      const int ix = idx / kb, q = idx % kb;
+    for (int ix = t >> 5; ix < cnt; ix += kBWarps) {
       const int z = S.srcmap[S.moved[ix]];
-      wutmp[(2 * ix) * kWU + q] = S.wsm[q * nw + z];
-      wutmp[(2 * ix + 1) * kWU + q] = S.usm[static_cast<size_t>(z) * S.ldu + q];
+      for (int q = t & 31; q < kb; q += 32) {
+        wutmp[(2 * ix) * kWU + q] = S.wsm[q * nw + z];
+        if (!kLean) wutmp[(2 * ix + 1) * kWU + q] = S.usm[q * nw + z];
+      }
     }
     __syncthreads();
     // write back: A in the interchanged order, the permutation, and W / U in
     // index order (from here on index = slot)
     const int mt0 = n - e;
-    pipelined_copy<8>(
-        cnt * mt0, [&](int idx) { return gbuf[static_cast<long long>(idx / mt0) * n + e + idx % mt0]; },
-        [&](int idx, double v) {
-          const int x = S.moved[idx / mt0], y = e + idx % mt0;
+    copy_rows<8>(
+        cnt, mt0, [&](int ix, int c) { return gbuf[static_cast<long long>(ix) * n + e + c]; },
+        [&](int ix, int c, double v) {
+          const int x = S.moved[ix], y = e + c;
           if (x < e) return;
           if (x <= y)
             A[static_cast<long long>(x) * lda + y] = v;
           else
             A[static_cast<long long>(y) * lda + x] = v;
         });
-    pipelined_copy<8>(
-        k0 * cnt, [&](int idx) { return gbuf2[static_cast<long long>(idx / cnt) * kCap + idx % cnt]; },
-        [&](int idx, double v) { A[static_cast<long long>(idx / cnt) * lda + S.moved[idx % cnt]] = v; });
+    copy_rows<8>(
+        k0, cnt, [&](int q, int ix) { return gbuf2[static_cast<long long>(q) * kCap + ix]; },
+        [&](int q, int ix, double v) { A[static_cast<long long>(q) * lda + S.moved[ix]] = v; });
     for (int ix = t; ix < cnt; ix += kBT) perm[S.moved[ix]] = permbuf[ix];
-    for (int idx = t; idx < cnt * kb; idx += kBT) {
-      const int ix = idx / kb, q = idx % kb;
+    for (int ix = t >> 5; ix < cnt; ix += kBWarps) {
       const int x = S.moved[ix];
-      S.wsm[q * nw + x] = wutmp[(2 * ix) * kWU + q];
-      S.usm[static_cast<size_t>(x) * S.ldu + q] = wutmp[(2 * ix + 1) * kWU + q];
+      for (int q = t & 31; q < kb; q += 32) {
+        S.wsm[q * nw + x] = wutmp[(2 * ix) * kWU + q];
+        if (!kLean) S.usm[q * nw + x] = wutmp[(2 * ix + 1) * kWU + q];
+      }
     }
     __syncthreads();
     // ---- compact factor rows [k0, e)
-    for (int idx = t; idx < kb * (n - k0); idx += kBT) {
-      const int q = idx / (n - k0), j = k0 + idx % (n - k0);
-      if (j < k0 + q) continue;
-      const int lj = j - k0;
-      double v;
-      if (j < e && q == lj)
-        v = S.dlog[2 * lj];
-      else if (j < e && q == lj - 1 && pt[j] == -2)
-        v = S.dlog[2 * q + 1];
-      else
-        v = S.usm[static_cast<size_t>(j) * S.ldu + q];
-      A[static_cast<long long>(k0 + q) * lda + j] = v;
+    for (int q = t >> 5; q < kb; q += kBWarps) {
+      double* row = A + static_cast<long long>(k0 + q) * lda;
+      for (int j = k0 + q + (t & 31); j < n; j += 32) {
+        const int lj = j - k0;
+        double v;
+        if (j < e && q == lj)
+          v = S.dlog[2 * lj];
+        else if (j < e && q == lj - 1 && pt[j] == -2)
+          v = S.dlog[2 * q + 1];
+        else
+          v = kLean ? u_value(S, q, j) : S.usm[q * nw + j];
+        row[j] = v;
+      }
     }
 
     // ---- trailing update of the upper triangle [e, n): A -= U^T W  (:706-744)
     const int mt = n - e;
     if (mt > 0 && kb > 0) {
+      if (kLean) __syncthreads();  // the compact rows are written
       if (kMode == BBK_UPDATE_FP64)
-        trailing_dmma(S, A, lda, n, e, kb);
+        trailing_dmma<kLean>(S, A, lda, n, e, kb);
       else
         trailing_simt<kMode>(S, A, lda, n, e, kb);
     }
@@ -749,8 +965,8 @@ __device__ double residual_one(const double* A, int n, int lda, const double* bv
   return den > 0.0 ? m[0] / den : (m[0] > 0.0 ? INFINITY : 0.0);
 }
 
-template <int kMode>
-__global__ void __launch_bounds__(kBT, 1) batched_kernel(BatchArgs B) {
+template <int kMode, int kC>
+__global__ void __launch_bounds__(kBT, 2) batched_kernel(BatchArgs B) {
   extern __shared__ double bsm[];
   __shared__ int s_item;
   double* gbuf = B.scratch + static_cast<long long>(blockIdx.x) * B.scratch_stride;
@@ -772,8 +988,19 @@ __global__ void __launch_bounds__(kBT, 1) batched_kernel(BatchArgs B) {
     double* X = B.x + I.rhs;
     int* perm = B.perm + I.piv;
     int* pt = B.ptype + I.piv;
-    Smem S = carve(bsm, n, I.b);
-    factor_one<kMode>(S, A, n, lda, I.b, perm, pt, gbuf, gbuf2, permbuf, wutmp);
+    Smem S;
+    bool lean = false;
+    if constexpr (kMode == BBK_UPDATE_FP64) lean = B.lean && batch_smem_bytes(n, I.b) > kHalfSmem;
+    if (lean) {
+      if constexpr (kMode == BBK_UPDATE_FP64) {
+        const int b = lean_block(n, I.b);
+        S = carve<true>(bsm, n, b);
+        factor_one<kMode, kC, true>(S, A, n, lda, b, perm, pt, gbuf, gbuf2, permbuf, wutmp);
+      }
+    } else {
+      S = carve<false>(bsm, n, I.b);
+      factor_one<kMode, kC, false>(S, A, n, lda, I.b, perm, pt, gbuf, gbuf2, permbuf, wutmp);
+    }
     // solve (the candidate-column buffer holds the vector)
     double* y = S.wcs;
     for (int i = threadIdx.x; i < n; i += kBT) {
@@ -819,23 +1046,37 @@ __global__ void __launch_bounds__(kBT, 1) batched_kernel(BatchArgs B) {
   }
 }
 
-constexpr size_t kHeaderBytes = 256;
-
-// Host-side record of planned workspaces (workspace -> count, largest order),
-// so a launch needs no device read.
-std::mutex g_plan_mu;
-std::map<const void*, std::pair<int, int>> g_plans;
-
-void batch_plan_record(const void* ws, int count, int max_n) {
-  std::lock_guard<std::mutex> lk(g_plan_mu);
-  g_plans[ws] = {count, max_n};
+// The kernel of an update mode for orders up to kC x kBT.
+template <int kC>
+const void* batched_kernel_of(int mode) {
+  static_assert(4 * kBT >= BBK_BATCH_MAX_N, "the largest order needs no more than four slots per thread");
+  return mode == BBK_UPDATE_FP64_ORDERED ? reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP64_ORDERED, kC>)
+         : mode == BBK_UPDATE_FP64       ? reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP64, kC>)
+                                         : reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP32, kC>);
 }
 
-bool batch_plan_lookup(const void* ws, int count, int* max_n) {
+constexpr size_t kHeaderBytes = 256;
+
+// Host-side record of planned workspaces, so a launch needs no device read:
+// the largest order, and the most shared memory an item takes, with one CTA
+// per SM and with two.
+struct BatchPlanInfo {
+  int count, max_n;
+  size_t smem, smem_half;
+};
+std::mutex g_plan_mu;
+std::map<const void*, BatchPlanInfo> g_plans;
+
+void batch_plan_record(const void* ws, const BatchPlanInfo& info) {
+  std::lock_guard<std::mutex> lk(g_plan_mu);
+  g_plans[ws] = info;
+}
+
+bool batch_plan_lookup(const void* ws, int count, BatchPlanInfo* info) {
   std::lock_guard<std::mutex> lk(g_plan_mu);
   auto it = g_plans.find(ws);
-  if (it == g_plans.end() || it->second.first != count) return false;
-  *max_n = it->second.second;
+  if (it == g_plans.end() || it->second.count != count) return false;
+  *info = it->second;
   return true;
 }
 
@@ -888,7 +1129,7 @@ using namespace bbk;
 
 extern "C" size_t bbk_batched_workspace_size(int count, int max_n) {
   if (count <= 0 || max_n <= 0 || max_n > BBK_BATCH_MAX_N) return 0;
-  return batch_layout(nullptr, count, max_n, device_sm_count()).bytes;
+  return batch_layout(nullptr, count, max_n, 2 * device_sm_count()).bytes;
 }
 
 extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const int* block_sizes,
@@ -897,6 +1138,7 @@ extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const in
   if (!items || !workspace) return set_error(BBK_ERR_INVALID_ARGUMENT, "null items or workspace");
   std::vector<BatchItemDev> v(count);
   int max_n = 0;
+  size_t smem = 0, smem_half = 0;
   for (int k = 0; k < count; ++k) {
     const bbk_batch_item& it = items[k];
     if (it.n <= 0 || it.n > BBK_BATCH_MAX_N)
@@ -907,12 +1149,14 @@ extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const in
     const int bkt = bucket_of(it.n);
     int b = (block_sizes && block_sizes[bkt] > 0) ? block_sizes[bkt] : default_block(bkt);
     b = std::min(std::min(b, kMaxB), it.n);
-    while (b > 1 && batch_smem_bytes(it.n, b) > kBatchSmem) --b;
-    if (batch_smem_bytes(it.n, b) > kBatchSmem)
+    while (b > 1 && batch_block_bytes(it.n, b) > kBatchSmem) --b;
+    if (batch_block_bytes(it.n, b) > kBatchSmem)
       return set_error(BBK_ERR_INVALID_ARGUMENT, "item %d: order %d does not fit shared memory", k, it.n);
     v[k] = BatchItemDev{it.n, it.lda, b, k, it.a, it.rhs, it.piv};
     if (chosen_blocks) chosen_blocks[k] = b;
     max_n = std::max(max_n, it.n);
+    smem = std::max(smem, batch_smem_bytes(it.n, b));
+    smem_half = std::max(smem_half, batch_half_bytes(it.n, b));
   }
   // largest first; ties keep the caller's order
   std::stable_sort(v.begin(), v.end(), [](const BatchItemDev& x, const BatchItemDev& y) { return x.n > y.n; });
@@ -928,7 +1172,7 @@ extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const in
   BBK_CUDA_TRY(cudaMemcpyAsync(L.items, v.data(), v.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice, s));
   BBK_CUDA_TRY(cudaStreamSynchronize(s));
   // the launch reads these back without a device round trip
-  batch_plan_record(workspace, count, max_n);
+  batch_plan_record(workspace, BatchPlanInfo{count, max_n, smem, smem_half});
   return BBK_OK;
 }
 
@@ -941,15 +1185,23 @@ extern "C" int bbk_batched_factor_solve(int count, double* a, const double* a_or
     return set_error(BBK_ERR_INVALID_ARGUMENT, "null buffer");
   if (update_mode != BBK_UPDATE_FP64 && update_mode != BBK_UPDATE_FP64_ORDERED && update_mode != BBK_UPDATE_FP32)
     return set_error(BBK_ERR_INVALID_ARGUMENT, "batched update mode must be FP64, FP64_ORDERED or FP32");
-  int max_n = 0;
-  if (!batch_plan_lookup(workspace, count, &max_n))
+  BatchPlanInfo plan{};
+  if (!batch_plan_lookup(workspace, count, &plan))
     return set_error(BBK_ERR_LOGIC, "workspace was not planned for %d items (call bbk_batched_plan)", count);
+  const int max_n = plan.max_n;
   int rc = check_device();
   if (rc) return rc;
-  const int grid = device_sm_count();
+  int grid = device_sm_count();
   BatchLayout L = batch_layout(workspace, count, max_n, grid);
   if (workspace_bytes < L.bytes)
     return set_error(BBK_ERR_WORKSPACE, "batched workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
+  // Two CTAs per SM where every item fits half of its shared memory (FP64:
+  // in the lean layout if need be) and the workspace has scratch for them.
+  const size_t two = batch_layout(nullptr, count, max_n, 2 * grid).bytes;
+  const bool lean =
+      update_mode == BBK_UPDATE_FP64 && plan.smem > kHalfSmem && plan.smem_half <= kHalfSmem && workspace_bytes >= two;
+  const size_t smem = lean ? plan.smem_half : plan.smem;
+  if (smem <= kHalfSmem && workspace_bytes >= two) grid *= 2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BatchArgs B{};
   B.count = count;
@@ -967,26 +1219,28 @@ extern "C" int bbk_batched_factor_solve(int count, double* a, const double* a_or
   B.scratch = L.scratch;
   B.scratch_stride = L.scratch_stride;
   B.max_n = max_n;
+  B.lean = lean;
   BBK_CUDA_TRY(cudaMemsetAsync(L.header, 0, sizeof(int), s));
-  const void* fn = update_mode == BBK_UPDATE_FP64_ORDERED
-                       ? reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP64_ORDERED>)
-                       : update_mode == BBK_UPDATE_FP64 ? reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP64>)
-                                                        : reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP32>);
+  const void* fn = max_n <= kBT       ? batched_kernel_of<1>(update_mode)
+                   : max_n <= 2 * kBT ? batched_kernel_of<2>(update_mode)
+                                      : batched_kernel_of<4>(update_mode);
   {
-    // once per device and mode, so a later call can run under stream capture
+    // once per device for every kernel, so a later call can run under stream capture
     static std::mutex mu;
-    static bool done[3][64] = {};
+    static bool done[64] = {};
     int dev = 0;
     BBK_CUDA_TRY(cudaGetDevice(&dev));
-    const int mi = update_mode == BBK_UPDATE_FP64_ORDERED ? 0 : update_mode == BBK_UPDATE_FP64 ? 1 : 2;
     std::lock_guard<std::mutex> lk(mu);
-    if (dev < 0 || dev >= 64 || !done[mi][dev]) {
-      BBK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBatchSmem)));
-      if (dev >= 0 && dev < 64) done[mi][dev] = true;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+      for (int mode : {BBK_UPDATE_FP64_ORDERED, BBK_UPDATE_FP64, BBK_UPDATE_FP32})
+        for (const void* k : {batched_kernel_of<1>(mode), batched_kernel_of<2>(mode), batched_kernel_of<4>(mode)})
+          BBK_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(kBatchSmem)));
+      if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
   void* kargs[] = {&B};
-  BBK_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(kBT), kargs, kBatchSmem, s));
+  BBK_CUDA_TRY(cudaLaunchKernel(fn, dim3(std::min(grid, count)), dim3(kBT), kargs, smem, s));
   count_launch();
   return BBK_OK;
 }

@@ -100,8 +100,9 @@ __device__ __forceinline__ double div_or_zero(double x, double den) {
 // from the first part's result is the same sum bit for bit).  The products
 // do not depend on the running sum: each batch of eight is loaded and
 // multiplied while the previous batch is being added.
-template <typename WGet>
-__device__ __forceinline__ double ordered_dot_range(double acc, const double* c, int q0, int q1, WGet&& w) {
+// (`c` is an array or anything indexed like one.)
+template <typename Coef, typename WGet>
+__device__ __forceinline__ double ordered_dot_range(double acc, const Coef& c, int q0, int q1, WGet&& w) {
   int q = q0;
   if (q1 - q0 >= 8) {
     double cur[8];
@@ -123,8 +124,8 @@ __device__ __forceinline__ double ordered_dot_range(double acc, const double* c,
   return acc;
 }
 
-template <typename WGet>
-__device__ __forceinline__ double ordered_dot(const double* c, int count, WGet&& w) {
+template <typename Coef, typename WGet>
+__device__ __forceinline__ double ordered_dot(const Coef& c, int count, WGet&& w) {
   return ordered_dot_range(0.0, c, 0, count, w);
 }
 
@@ -204,8 +205,8 @@ __device__ __forceinline__ void split_dot2(const double* c1, const double* c2, i
 // combined pairwise: the same sum, reassociated, with an eighth of the
 // dependent-latency chain (update modes that do not reproduce the
 // reference's rounding).
-template <typename WGet>
-__device__ __forceinline__ double split_dot_range(const double* c, int q0, int q1, WGet&& w) {
+template <typename Coef, typename WGet>
+__device__ __forceinline__ double split_dot_range(const Coef& c, int q0, int q1, WGet&& w) {
   double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   int q = q0;
   for (; q + 8 <= q1; q += 8) {
@@ -218,8 +219,8 @@ __device__ __forceinline__ double split_dot_range(const double* c, int q0, int q
   return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
 }
 
-template <typename WGet>
-__device__ __forceinline__ double split_dot(const double* c, int count, WGet&& w) {
+template <typename Coef, typename WGet>
+__device__ __forceinline__ double split_dot(const Coef& c, int count, WGet&& w) {
   return split_dot_range(c, 0, count, w);
 }
 
