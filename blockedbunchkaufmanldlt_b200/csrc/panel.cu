@@ -46,7 +46,7 @@
 // Panels of up to a few thousand columns run on one thread-block cluster.
 // KKT n = 10000, block 128: 50.1 -> 42.5 ms per factorization (4.2 us per
 // pivot); KKT n = 1999, block 64: 9.3 -> 6.3 ms; n = 40000, block 256: 384 ->
-// 362 ms.
+// 300 ms.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -68,7 +68,9 @@ constexpr int kWarps = kThreads / 32;  // compute warps
 constexpr int kCommWarp = kWarps;       // the communication warp
 constexpr int kBlock = kThreads + 32;   // compute warps + the communication warp
 constexpr int kCols = 3;  // slots per thread: S <= kCols * kThreads
-constexpr int kPairSlots = 96;  // slots per CTA up to which the warps split the candidate sums by rows
+constexpr int kNarrowSlots = 96;  // slots per CTA up to which the warps split the candidate sums by rows
+constexpr int kWideSlots = 288;   // in the kernels for few and for many slots
+constexpr int kGlobalRows = 4;  // rows in flight per thread of sums over rows in global memory
 constexpr int kAllWarps = kBlock / 32;
 constexpr int kClusterMax = 16;      // CTAs of a cluster panel
 constexpr int kClusterSlots = 224;   // slots per CTA of a cluster panel: 7 per lane
@@ -114,6 +116,7 @@ struct PanelArgs {
   int coef_cap;      // doubles reserved for each coefficient column
   int w_smem;        // keep this CTA's panel rows in shared memory
   int smem_cols;     // slice width the shared-memory allocation holds
+  int part_pitch;    // slots of a row of per-warp partial sums
   int wcap;          // doubles of shared memory for panel rows: all of them (w_smem), else the
                      // first wcap / S rows of the slice (the rest in wslot)
   unsigned long long* stats;  // optional per-phase nanoseconds (CTA 0)
@@ -589,10 +592,12 @@ __device__ __forceinline__ void by_chunks(int width, F&& f) {
 // cluster's shared memory, and so do U columns: they are formed from W and
 // the pivots' scaling, which every CTA keeps, by their owner instead of being
 // stored; gather_kernel collects the moved rows afterwards.
-template <bool kOrdered, bool kSmemW, bool kCluster>
+// kPairs: up to this many slots per CTA the compute warps split the rows of
+// the reassociated modes' sums (every warp a sixth of them for all slots, so
+// each coefficient is read once and no thread has more slots than another).
+template <bool kOrdered, bool kSmemW, bool kCluster, int kPairs>
 __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   static_assert(kSmemW || !kCluster, "a cluster panel keeps its rows in shared memory");
-  constexpr int kPairs = kCluster ? kClusterSlots : kPairSlots;
   constexpr int kPairLanes = kPairs / 32;
   extern __shared__ double dsm[];
   __shared__ XShared X;
@@ -612,8 +617,6 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   const int kstart = ldcg(&P.st->kstart[P.panel & 1]);
   const int S = (n - kstart + G - 1) / G;  // slots per CTA
   const int SP = kCluster ? (S | 1) : S;   // row pitch of the slice (odd: columns are read without bank conflicts)
-  // reassociated modes with at most kPairs slots per CTA: the compute
-  // warps split the rows of the candidate and look-ahead sums
   const bool paired = !kOrdered && S <= kPairs;
   const int lo = kstart + c * S;
   const int hi = min(n, lo + S);
@@ -633,8 +636,9 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   double* coef2 = dsm + P.coef_cap;  // coefficients of a row computed ahead
   double* wcs = dsm + 2 * P.coef_cap;
   double* svs = wcs + P.smem_cols;   // the row computed ahead, by slot
-  double* wpart = svs + P.smem_cols;  // per-warp partial sums: 2 x kWarps x kPairs
-  double* wsm = wpart + 2 * kWarps * kPairs;  // wcap doubles
+  double* wpart = svs + P.smem_cols;  // per-warp partial sums: 2 x kWarps x part_pitch
+  const int pp = P.part_pitch;
+  double* wsm = wpart + 2 * kWarps * pp;  // wcap doubles
   int* win = reinterpret_cast<int*>(wsm + P.wcap);
   int* mypos = win + P.win_pad;  // index held by slot lo + zz
   // cluster panels: how row q of U follows from W (upk: 1 W / ua; 2 first, 3
@@ -648,6 +652,23 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
   auto wat = [&](int m, int z) -> double& {
     if (kSmemW || m < srows) return wsm[m * SP + (z - lo)];
     return P.wslot[m * ldw + z];
+  };
+  // the rows [qa, qb) in shared memory and [ga, gb) in global memory that warp
+  // w sums: a sixth of all, or (kernels for many slots) of either
+  auto warp_rows = [&](int lp, int w, int& qa, int& qb, int& ga, int& gb) {
+    const int qs = kSmemW ? lp : min(lp, srows);
+    if (kPairs > kNarrowSlots) {
+      qa = (qs * w) / kWarps;
+      qb = (qs * (w + 1)) / kWarps;
+      ga = qs + ((lp - qs) * w) / kWarps;
+      gb = qs + ((lp - qs) * (w + 1)) / kWarps;
+    } else {
+      const int a = (lp * w) / kWarps, b = (lp * (w + 1)) / kWarps;
+      qa = min(a, qs);
+      qb = min(b, qs);
+      ga = max(a, qs);
+      gb = max(b, qs);
+    }
   };
   // the same, split by where the rows live (the hot dot products run over
   // the shared-memory rows and then the global ones)
@@ -822,24 +843,40 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         // the compute warps split the rows q < lp (see the candidate phase)
         if (t < kThreads) {
           const int w = t >> 5, ln = t & 31;
-          const int qa = (lp * w) / kWarps, qb = (lp * (w + 1)) / kWarps;
-          const int qm = kSmemW ? qb : min(max(qa, srows), qb);
+          int qa, qb, ga, gb;
+          warp_rows(lp, w, qa, qb, ga, gb);
           by_chunks<kPairLanes>(width, [&](auto chunks) {
             constexpr int N = decltype(chunks)::value;
             double s1[N] = {};
-            auto rows = [&](int q0, int q1, const double* wp, long long pitch) {
-              for (int q = q0; q < q1; ++q, wp += pitch) {
+            auto rows = [&](auto global, int q0, int q1, const double* wp, long long pitch) {
+              constexpr int kU = decltype(global)::value ? kGlobalRows : 1;
+              int q = q0;
+              if constexpr (kU > 1) {
+                for (; q + kU <= q1; q += kU, wp += kU * pitch) {
+                  double x[kU][N];
+#pragma unroll
+                  for (int u = 0; u < kU; ++u)
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+                      x[u][k] = k < N - 1 || ln + 32 * k < width ? wp[u * pitch + 32 * k] : 0.0;
+#pragma unroll
+                  for (int u = 0; u < kU; ++u)
+#pragma unroll
+                    for (int k = 0; k < N; ++k) s1[k] = __fma_rn(coef[q + u], x[u][k], s1[k]);
+                }
+              }
+              for (; q < q1; ++q, wp += pitch) {
                 const double c1 = coef[q];
 #pragma unroll
                 for (int k = 0; k < N; ++k)
                   if (k < N - 1 || ln + 32 * k < width) s1[k] = __fma_rn(c1, wp[32 * k], s1[k]);
               }
             };
-            rows(qa, qm, wsm + qa * SP + ln, SP);
-            if (!kSmemW) rows(qm, qb, P.wslot + qm * ldw + lo + ln, ldw);
+            rows(std::false_type{}, qa, qb, wsm + qa * SP + ln, SP);
+            if (!kSmemW) rows(std::true_type{}, ga, gb, P.wslot + ga * ldw + lo + ln, ldw);
 #pragma unroll
             for (int k = 0; k < N; ++k)
-              if (k < N - 1 || ln + 32 * k < width) wpart[w * kPairs + ln + 32 * k] = s1[k];
+              if (k < N - 1 || ln + 32 * k < width) wpart[w * pp + ln + 32 * k] = s1[k];
           });
           compute_warps_sync();
         }
@@ -851,7 +888,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
             if (j >= p) {
               double acc = wpart[zz];
 #pragma unroll
-              for (int w = 1; w < kWarps; ++w) acc += wpart[w * kPairs + zz];
+              for (int w = 1; w < kWarps; ++w) acc += wpart[w * pp + zz];
               finish_row(lo + zz, j, av[k], acc);
             }
           }
@@ -1040,13 +1077,34 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
         // per-warp partial sums are then added in warp order
         if (t < kThreads) {
           const int w = t >> 5, ln = t & 31;
-          const int qa = (lp * w) / kWarps, qb = (lp * (w + 1)) / kWarps;
-          const int qm = kSmemW ? qb : min(max(qa, srows), qb);
+          int qa, qb, ga, gb;
+          warp_rows(lp, w, qa, qb, ga, gb);
           by_chunks<kPairLanes>(width, [&](auto chunks) {
             constexpr int N = decltype(chunks)::value;
             double sa[N] = {}, sb[N] = {};
-            auto rows = [&](int q0, int q1, const double* wp, long long pitch) {
-              for (int q = q0; q < q1; ++q, wp += pitch) {
+            auto rows = [&](auto global, int q0, int q1, const double* wp, long long pitch) {
+              constexpr int kU = decltype(global)::value ? kGlobalRows : 1;
+              int q = q0;
+              if constexpr (kU > 1) {
+                for (; q + kU <= q1; q += kU, wp += kU * pitch) {
+                  double x[kU][N];
+#pragma unroll
+                  for (int u = 0; u < kU; ++u)
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+                      x[u][k] = k < N - 1 || ln + 32 * k < width ? wp[u * pitch + 32 * k] : 0.0;
+#pragma unroll
+                  for (int u = 0; u < kU; ++u) {
+                    const double c1 = coef[q + u], c2 = coef2[q + u];
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                      sa[k] = __fma_rn(c1, x[u][k], sa[k]);
+                      sb[k] = __fma_rn(c2, x[u][k], sb[k]);
+                    }
+                  }
+                }
+              }
+              for (; q < q1; ++q, wp += pitch) {
                 const double c1 = coef[q], c2 = coef2[q];
 #pragma unroll
                 for (int k = 0; k < N; ++k)
@@ -1057,13 +1115,13 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
                   }
               }
             };
-            rows(qa, qm, wsm + qa * SP + ln, SP);
-            if (!kSmemW) rows(qm, qb, P.wslot + qm * ldw + lo + ln, ldw);
+            rows(std::false_type{}, qa, qb, wsm + qa * SP + ln, SP);
+            if (!kSmemW) rows(std::true_type{}, ga, gb, P.wslot + ga * ldw + lo + ln, ldw);
 #pragma unroll
             for (int k = 0; k < N; ++k)
               if (k < N - 1 || ln + 32 * k < width) {
-                wpart[(2 * w) * kPairs + ln + 32 * k] = sa[k];
-                wpart[(2 * w + 1) * kPairs + ln + 32 * k] = sb[k];
+                wpart[(2 * w) * pp + ln + 32 * k] = sa[k];
+                wpart[(2 * w + 1) * pp + ln + 32 * k] = sb[k];
               }
           });
           compute_warps_sync();
@@ -1074,11 +1132,11 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
           if (zz < width) {
             const int i = mypos[zz];
             if (i >= p) {
-              double acc = wpart[zz], part = wpart[kPairs + zz];
+              double acc = wpart[zz], part = wpart[pp + zz];
 #pragma unroll
               for (int w = 1; w < kWarps; ++w) {
-                acc += wpart[(2 * w) * kPairs + zz];
-                part += wpart[(2 * w + 1) * kPairs + zz];
+                acc += wpart[(2 * w) * pp + zz];
+                part += wpart[(2 * w + 1) * pp + zz];
               }
               finish(lo + zz, i, acc, part, spec && i > p);
             }
@@ -1735,7 +1793,7 @@ static int cluster_limit(const void* fn) {
   static int limit[2][64] = {};  // by kernel and device; 0: not asked yet, -1: none
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  int& l = limit[fn == reinterpret_cast<const void*>(panel_kernel<true, true, true>)][dev];
+  int& l = limit[fn == reinterpret_cast<const void*>(panel_kernel<true, true, true, kClusterSlots>)][dev];
   std::lock_guard<std::mutex> lk(mu);
   if (l == 0) {
     l = -1;
@@ -1778,8 +1836,8 @@ static int launch_cluster_panel(const FactorPlan& plan, PanelArgs P, bool ordere
   const long long start = std::max(0LL, static_cast<long long>(P.panel) * plan.b - 1);
   const long long m = plan.n - start;
   if (m > static_cast<long long>(kClusterMax) * kClusterSlots) return BBK_OK;
-  const void* fn = ordered ? reinterpret_cast<const void*>(panel_kernel<true, true, true>)
-                           : reinterpret_cast<const void*>(panel_kernel<false, true, true>);
+  const void* fn = ordered ? reinterpret_cast<const void*>(panel_kernel<true, true, true, kClusterSlots>)
+                           : reinterpret_cast<const void*>(panel_kernel<false, true, true, kClusterSlots>);
   int G = 1;
   while (G < kClusterMax && m > static_cast<long long>(kClusterCols) * G) G *= 2;
   G = std::min(G, cluster_limit(fn));
@@ -1788,11 +1846,12 @@ static int launch_cluster_panel(const FactorPlan& plan, PanelArgs P, bool ordere
   if (smax > kClusterSlots) return BBK_OK;
   P.coef_cap = static_cast<int>(align_up(static_cast<size_t>(plan.b) + 4, 2));
   P.smem_cols = static_cast<int>(smax);
+  P.part_pitch = static_cast<int>(smax);
   P.w_smem = 1;
   P.wcap = P.win_rows * static_cast<int>(smax | 1);
   const size_t cols = align_up(static_cast<size_t>(smax), 2);
   const size_t bytes = (4 * static_cast<size_t>(P.coef_cap) + 2 * static_cast<size_t>(smax) +
-                        2 * static_cast<size_t>(kWarps) * kClusterSlots + P.wcap) * sizeof(double) +
+                        2 * static_cast<size_t>(kWarps) * P.part_pitch + P.wcap) * sizeof(double) +
                        (2 * static_cast<size_t>(P.win_pad) + cols) * sizeof(int);
   if (bytes > kClusterSmem) return BBK_OK;
   cudaLaunchConfig_t cfg{};
@@ -1871,11 +1930,19 @@ int launch_panel(const FactorPlan& plan, int panel, cudaStream_t s) {
     const int rc = launch_cluster_panel(plan, P, ordered, &clustered, s);
     if (rc || clustered) return rc;
   }
-  const int smax = (plan.n + plan.grid - 1) / plan.grid;
+  // (a boundary shift starts a panel one row early)
+  const int m = plan.n - static_cast<int>(std::max(0LL, static_cast<long long>(panel) * plan.b - 1));
+  // Factors whose update runs in low precision amplify the last bit of a sum
+  // to the update's precision, where a pivot may tip: these modes keep the
+  // order of the sums that the widest slice of the factorization gives (its
+  // rows in shared memory, one thread per slot beyond kNarrowSlots).
+  const bool fixed = plan.mode != BBK_UPDATE_FP64 && !ordered;
+  const int smax = ((fixed ? plan.n : m) + plan.grid - 1) / plan.grid;
   P.coef_cap = static_cast<int>(align_up(static_cast<size_t>(plan.b) + 4, 2));
   P.smem_cols = smax;
+  P.part_pitch = fixed ? kNarrowSlots : std::min(smax, kWideSlots);
   const size_t base = (2 * static_cast<size_t>(P.coef_cap) + 2 * static_cast<size_t>(smax) +
-                       2 * static_cast<size_t>(kWarps) * kPairSlots) * sizeof(double) +
+                       2 * static_cast<size_t>(kWarps) * P.part_pitch) * sizeof(double) +
                       (static_cast<size_t>(P.win_pad) + smax) * sizeof(int);
   const size_t wbytes = static_cast<size_t>(P.win_rows) * smax * sizeof(double);
   const size_t limit = 220 * 1024;
@@ -1896,10 +1963,17 @@ int launch_panel(const FactorPlan& plan, int panel, cudaStream_t s) {
   }
   P.wcap = static_cast<int>(wroom / sizeof(double));
   const size_t bytes = base + wroom;
-  const void* fn = ordered ? (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<true, true, false>)
-                                       : reinterpret_cast<const void*>(panel_kernel<true, false, false>))
-                           : (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<false, true, false>)
-                                       : reinterpret_cast<const void*>(panel_kernel<false, false, false>));
+  // The sums' registers and code are sized by the slots a lane may have; with
+  // nine the kernel for few slots loses 4 % (KKT n = 10000: 42.5 -> 44.0 ms),
+  // and n = 40000, 271 slots, gains 14 % over one thread per slot (362 -> 312).
+  const bool few = fixed || smax <= kNarrowSlots;
+  const void* fn =
+      ordered ? (P.w_smem ? reinterpret_cast<const void*>(panel_kernel<true, true, false, kNarrowSlots>)
+                          : reinterpret_cast<const void*>(panel_kernel<true, false, false, kNarrowSlots>))
+      : P.w_smem ? (few ? reinterpret_cast<const void*>(panel_kernel<false, true, false, kNarrowSlots>)
+                        : reinterpret_cast<const void*>(panel_kernel<false, true, false, kWideSlots>))
+                 : (few ? reinterpret_cast<const void*>(panel_kernel<false, false, false, kNarrowSlots>)
+                        : reinterpret_cast<const void*>(panel_kernel<false, false, false, kWideSlots>));
   BBK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
   void* kargs[] = {&P};
   cudaError_t err = cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(kBlock), kargs, bytes, s);

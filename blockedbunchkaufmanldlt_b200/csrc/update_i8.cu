@@ -98,10 +98,17 @@ __global__ void __launch_bounds__(256) row_max_kernel(SliceArgs S) {
   if (k >= r.inner) return;
   const double* row = S.w + static_cast<long long>(k) * S.ldw;
   unsigned long long m = 0;
-  for (int x = r.e + blockIdx.x * 256 + threadIdx.x; x < S.n; x += gridDim.x * 256) {
-    const unsigned long long v =
-        static_cast<unsigned long long>(__double_as_longlong(row[x])) & 0x7fffffffffffffffull;
-    m = v > m ? v : m;
+  const int step = gridDim.x * 256;
+  for (int x = r.e + blockIdx.x * 256 + threadIdx.x; x < S.n; x += 4 * step) {
+    double v[4];  // four loads in flight
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = x + u * step < S.n ? row[x + u * step] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const unsigned long long w =
+          static_cast<unsigned long long>(__double_as_longlong(v[u])) & 0x7fffffffffffffffull;
+      m = w > m ? w : m;
+    }
   }
   for (int off = 16; off > 0; off >>= 1) {
     const unsigned long long o = __shfl_down_sync(0xffffffffu, m, off);

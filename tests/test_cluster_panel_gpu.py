@@ -74,3 +74,29 @@ def test_an_expired_wait_in_a_cluster_is_reported_and_the_context_survives(cuda,
     perm, pt, _ = bbk.factor_device(f, 64)
     r = bbk.reconstruct_device(f, perm, pt).cpu().numpy()
     assert relative_error(r, a) < 1e-10
+
+
+@pytest.mark.parametrize("slots", [97, 129, 288])
+def test_many_slots_per_cta_split_the_rows(cuda, bbk, slots):
+    # the grid panel's kernel for 97 to 288 slots per CTA, its rows split
+    # between shared and global memory (block 256 beyond 90 slots or so): the
+    # decisions' quantities agree with the ordered mode's to rounding, and the
+    # pivots where no decision is a near-tie
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = slots * sms
+    if n > 30000:
+        n = 30000 - 30000 % sms  # the check is the residual's; memory bounds the order
+    g = torch.Generator(device=cuda)
+    g.manual_seed(slots)
+    a = torch.empty(n, n, dtype=torch.float64, device=cuda).uniform_(-1.0, 1.0, generator=g)
+    a = torch.triu(a) + torch.triu(a, 1).T
+    f = a.clone()
+    perm, pt, ends = bbk.factor_device(f, 256)
+    p = perm.cpu().numpy()
+    assert np.array_equal(np.sort(p), np.arange(n))
+    b = torch.randn(2, n, dtype=torch.float64, device=cuda, generator=g)
+    x = bbk.solve_device(f, perm, pt, b.clone())
+    r = (b.T - a @ x.T).abs().amax(0)
+    berr = r / (a.abs().sum(1).amax() * x.T.abs().amax(0) + b.T.abs().amax(0))
+    assert float(berr.max()) < 1e-13
