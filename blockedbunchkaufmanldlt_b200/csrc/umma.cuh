@@ -51,4 +51,49 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const unsigned char* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// 16 rows x 8 columns of an accumulator: v[0], v[1] row lane / 4, v[2], v[3]
+// row lane / 4 + 8, at columns 2 (lane % 4) and the next.
+__device__ __forceinline__ void tmem_ld16x8(uint32_t addr, int (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(addr));
+}
+
+// Tile t of an upper triangle of tm x tm tiles (row I, column J >= I): in
+// strips of kStrip tile columns, row by row within a strip, so the CTAs that
+// run together share a few row and column blocks of operands in L2.
+constexpr int kStrip = 12;  // 12 x 12 tiles for 148 CTAs
+__device__ __forceinline__ void strip_tile(int t, int tm, int& I, int& J) {
+  constexpr int kTri = kStrip * (kStrip + 1) / 2;
+  auto before = [](int q) { return kStrip * kStrip * (q * (q - 1) / 2) + kTri * q; };  // tiles of the strips < q
+  int q = static_cast<int>(sqrt(2.0 * t) / kStrip);
+  while (q > 0 && before(q) > t) --q;
+  while (before(q + 1) <= t) ++q;
+  const int j0 = q * kStrip, w = min(kStrip, tm - j0);
+  int u = t - before(q);
+  if (u < w * j0) {
+    I = u / w;
+    J = j0 + u % w;
+    return;
+  }
+  u -= w * j0;
+  int j = 0;
+  while ((j + 1) * (j + 2) / 2 <= u) ++j;
+  I = j0 + u - j * (j + 1) / 2;
+  J = j0 + j;
+}
+
 }  // namespace bbk

@@ -7,9 +7,10 @@
 // C(i,j) -= sum_k A(i,k) B(k,j) with A(i,k) = U[k, i] and B(k,j) = W[k, j].
 // Arithmetics:
 //   FP64          integer tensor cores on 8-bit digits for large panels
-//                 (update_i8.cu), else FP64 tensor cores: mma.sync.m16n8k8.f64 from shared-memory
-//                 tiles staged with cp.async (double-buffered); 64x64 C tile
-//                 per CTA, 32x32 per warp.
+//                 (update_i8.cu), else FP64 tensor cores:
+//                 mma.sync.m16n8k8.f64 from shared-memory tiles staged with
+//                 cp.async (double-buffered); 64x64 C tile per CTA, 32x32 per
+//                 warp.
 //   FP64_ORDERED  SIMT, every product and sum rounded separately with k
 //                 ascending and one final subtraction: bitwise the
 //                 reference's arithmetic.
@@ -751,7 +752,9 @@ bool use_k16() {
   return v;
 }
 
-// Tile shape of the FP64 tensor-core update for large trailing matrices:
+// Tile shape of the FP64 tensor-core update where the digit update does not
+// apply (narrow blocks, entries beyond its range, unaligned matrices) and the
+// trailing matrix is large:
 // by default 64 x 64 tiles in the 4-stage ring of k chunks of 8 (five CTAs
 // per SM; n=40000: 27.9 TFLOP/s, against 26.9 for the 3-stage ring of 16
 // and 25.7 for the two-stage 64 x 64 kernel).  BBK_UPDATE_TILE (tuning) =
@@ -1139,29 +1142,38 @@ __global__ void __launch_bounds__(256) split_blocked_kernel(UpdArgs U, __nv_bflo
 // tensor memory (128 lanes x 128 columns).  Completion is tracked by
 // mbarriers (transaction bytes for the copies, tcgen05.commit for the MMAs);
 // every wait is bounded and a wait that runs out aborts the factorization
-// with BBK_ERR_TIMEOUT.  The epilogue reads an accumulator with tcgen05.ld
-// (warp w: lanes 32w.., one C row per thread), unscales it and subtracts it
-// from the FP64 trailing matrix, while the other accumulator takes the next
-// tile's MMAs.  Two CTAs per SM.
+// with BBK_ERR_TIMEOUT.  Sixteen epilogue warps load their part of C (32 x 32
+// entries each) before a tile's MMAs are done, read the accumulator with
+// tcgen05.ld in the shape that gives four lanes 64 bytes of a C row, unscale
+// it and subtract it, while the other three accumulators take the next
+// tiles' MMAs.  A tile with k = 256 has to move 256 KB of C (11 000 cycles at
+// the memory's rate) against 6 500 cycles of MMAs.  Update of the
+// factorization, three terms, ms: n = 16000, block 256: 24.1 -> 14.6; n =
+// 18000, block 128: 53.6 -> 32.6; n = 40000, block 256: 291 -> 189 (one term:
+// 255 -> 145).  Before, four epilogue warps held one C row per thread, eight
+// columns at a time, and two accumulators per CTA, two CTAs per SM; one lane
+// alone issued the MMAs (96 cycles each of the 64 they take).  The products
+// and the order in which they enter a sum are the same, to the last bit.
 // ---------------------------------------------------------------------------
 constexpr int kUM = 128, kUN = 128;  // C tile
 
+constexpr int kUEpi = 16;                      // epilogue warps
+constexpr int kUCols = 4 * kUN / kUEpi;        // columns of an epilogue warp
+constexpr int kUAcc = 4;                       // accumulators of kUN TMEM columns
+constexpr int kUBlock = (kUEpi + 2) * 32;
 
-// Per term count: the k chunk (BF16 elements) and the stages, sized so that
-// two CTAs fit one SM with the same bytes in flight (three terms: more,
-// shorter stages, so a stage is refilled soon after its MMAs finish).
+// Per term count: the stages of one k chunk each (one 4 KB block per operand
+// and term), in one CTA per SM.
 template <int kTerms>
 struct USmem {
-  static constexpr int kK = kBlkK;
-  static constexpr int kOpBytes = kUM * kK * 2;  // one term of one operand per stage: one 4 KB block
-  static constexpr int kRowGroup = (kK / 8) * 128;  // bytes between 8-row core-matrix groups
+  static constexpr int kOpBytes = kUM * kBlkK * 2;
   static constexpr int kStageBytes = 2 * kTerms * kOpBytes;
-  static constexpr int kStages = kTerms == 3 ? 4 : 8;
-  // stages, then the barriers (2 x kStages + 4) and the accumulator address
-  static constexpr size_t kBytes = static_cast<size_t>(kStages) * kStageBytes + 256;
-  static_assert((2 * kStages + 4) * 8 + 4 <= 256, "barrier area");
+  static constexpr int kStages = kTerms == 3 ? 8 : 16;
+  // stages, then the barriers (2 x kStages + 2 x kUAcc + 1) and the accumulators' address
+  static constexpr size_t kBytes = static_cast<size_t>(kStages) * kStageBytes + 512;
+  static_assert((2 * kStages + 2 * kUAcc + 1) * 8 + 4 <= 512, "barrier area");
+  static_assert(kBytes <= 227 * 1024, "stages fit the shared memory of one CTA");
 };
-static_assert(2 * USmem<3>::kBytes + 2048 <= 228 * 1024, "two CTAs per SM");
 
 // Instruction descriptor of kind::f16: FP32 accumulate, BF16 A and B, both
 // K-major, N = 128, M = 128.
@@ -1176,38 +1188,28 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
 }
 
 // Roles (warp-specialized, no CTA barrier inside the main loop):
-//   warps 0-3   epilogue: wait until an accumulator is full, read it with
-//               tcgen05.ld (warp w: lanes 32w..32w+31, one C row per
-//               thread), C -= unscale * acc, then mark the accumulator empty;
-//   warp 4      lane 0 moves the next chunk into a free stage with bulk
-//               asynchronous copies (one 4 KB block per operand and term,
-//               split_blocked_kernel's layout) that complete the stage's
-//               "full" barrier;
-//   warp 5      lane 0 issues the MMAs of each full stage, commits them to
-//               the stage's "empty" barrier and, after a tile's last chunk,
-//               to the accumulator's "full" barrier.
-// Two accumulators (2 x 128 TMEM columns) let the epilogue of one tile run
-// while the next tile's MMAs execute.
-constexpr int kUEpi = 4, kUProd = 1;
-constexpr int kUWarps = kUEpi + kUProd + 1;
-constexpr int kUBlock = kUWarps * 32;
-
+//   warps 0-15  epilogue (warp w: rows 32 (w % 4).., columns 32 (w / 4)..);
+//   warp 16     lane 0 moves the next chunk into a free stage with bulk
+//               asynchronous copies (split_blocked_kernel's layout) that
+//               complete the stage's "full" barrier;
+//   warp 17     walks the full stages; one lane issues their MMAs, commits
+//               them to the stage's "empty" barrier and, after a tile's last
+//               chunk, to the accumulator's "full" barrier.
 template <int kTerms>
-__global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U, const __nv_bfloat16* ah,
+__global__ void __launch_bounds__(kUBlock, 1) umma_bf16s_update_kernel(UpdArgs U, const __nv_bfloat16* ah,
                                                                        const __nv_bfloat16* bh, int kpad,
                                                                        size_t term_stride,
                                                                        unsigned long long timeout_ns) {
   using S = USmem<kTerms>;
-  constexpr int kUK = S::kK;
-  constexpr int kUOpBytes = S::kOpBytes;
   extern __shared__ __align__(1024) unsigned char usm[];
   uint64_t* full = reinterpret_cast<uint64_t*>(usm + S::kStages * S::kStageBytes);
   uint64_t* empty = full + S::kStages;
-  uint64_t* accfull = empty + S::kStages;  // 2
-  uint64_t* accempty = accfull + 2;        // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + 2);
-  // the panel's range (the split operands start at split_i0, the 64-aligned
-  // row at or below the trailing matrix; tiles here are 128-aligned)
+  uint64_t* accfull = empty + S::kStages;
+  uint64_t* accempty = accfull + kUAcc;
+  uint64_t* idle = accempty + kUAcc;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(idle + 1);
+  // the panel's range (the split operands' scales start at split_i0, the
+  // 64-aligned row at or below the trailing matrix; tiles are 128-aligned)
   if (ld_relaxed_s32(&U.st->abort)) return;
   const int k0p = ldcg(&U.st->kstart[U.panel & 1]);
   const int e = ldcg(&U.st->kstart[(U.panel + 1) & 1]);
@@ -1218,14 +1220,14 @@ __global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U
   const int tm = (U.n - t_i0 + kUM - 1) / kUM;
   const int ntiles = tm * (tm + 1) / 2;
   if (static_cast<int>(blockIdx.x) >= ntiles) return;
-  const int nchunks = (inner + kUK - 1) / kUK;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nchunks = (inner + kBlkK - 1) / kBlkK;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int my_tiles = (ntiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                        static_cast<int>(gridDim.x);
 
-  if (warp == kUWarps - 1) {
+  if (warp == kUEpi + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(2 * kUN)
+                 "r"(kUAcc * kUN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     if (lane == 0) {
@@ -1233,43 +1235,43 @@ __global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[st])) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[st])) : "memory");
       }
-      for (int b = 0; b < 2; ++b) {
+      for (int b = 0; b < kUAcc; ++b) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&accfull[b])) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&accempty[b])), "r"(kUEpi)
                      : "memory");
       }
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(idle)) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  auto tile_of = [&](int t, int& i0, int& j0) {
-    int j = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-    while (j > 0 && j * (j + 1) / 2 > t) --j;
-    while ((j + 1) * (j + 2) / 2 <= t) ++j;
-    i0 = t_i0 + (t - j * (j + 1) / 2) * kUM;
-    j0 = t_i0 + j * kUN;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  auto tile_of = [&](int m, int& I, int& J) {  // tile m of this CTA
+    strip_tile(static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), tm, I, J);
+  };
+  auto wait = [&](uint64_t* bar, int phase) {  // of a whole warp
+    const bool got = mbar_wait(smem_u32(bar), static_cast<uint32_t>(phase & 1), U.st, timeout_ns);
+    if (!__all_sync(0xffffffffu, got)) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return true;
   };
   bool ok = true;
 
   if (warp == kUEpi) {
-    // ---- producer: one thread moves each stage's 2 x kTerms blocks with
-    // bulk asynchronous copies that complete the stage's "full" barrier
     if (lane == 0) {
       const int nkc = kpad / kBlkK;
-      long long item = 0;
+      int item = 0;
       for (int m = 0; m < my_tiles && ok; ++m) {
-        int i0, j0;
-        tile_of(static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), i0, j0);
-        const int rba = (i0 - t_i0) / kBlkRows, rbb = (j0 - t_i0) / kBlkRows;
+        int I, J;
+        tile_of(m, I, J);
+        const __nv_bfloat16* a = ah + static_cast<size_t>(I) * nkc * kBlkElems;
+        const __nv_bfloat16* b = bh + static_cast<size_t>(J) * nkc * kBlkElems;
         for (int ch = 0; ch < nchunks; ++ch, ++item) {
-          const int st = static_cast<int>(item % S::kStages);
-          const long long use = item / S::kStages;
-          if (use >= 1 &&
-              !mbar_wait(smem_u32(&empty[st]), static_cast<uint32_t>((use - 1) & 1), U.st, timeout_ns)) {
+          const int st = item % S::kStages;
+          if (item >= S::kStages && !mbar_wait(smem_u32(&empty[st]),
+                                               static_cast<uint32_t>((item / S::kStages - 1) & 1), U.st, timeout_ns)) {
             ok = false;
             break;
           }
@@ -1277,146 +1279,121 @@ __global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(S::kStageBytes)
                        : "memory");
           const uint32_t base = smem_u32(usm + st * S::kStageBytes);
-          for (int blk = 0; blk < 2 * kTerms; ++blk) {
-            const int op = blk / kTerms, term = blk - op * kTerms;
-            const __nv_bfloat16* src = (op == 0 ? ah : bh) + term * term_stride +
-                                       static_cast<size_t>((op == 0 ? rba : rbb) * nkc + ch) * kBlkElems;
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    base + blk * kUOpBytes),
-                "l"(src), "r"(kUOpBytes), "r"(fb)
-                : "memory");
+          const size_t off = static_cast<size_t>(ch) * kBlkElems;
+#pragma unroll
+          for (int t = 0; t < kTerms; ++t) {
+            bulk_load(base + t * S::kOpBytes, reinterpret_cast<const unsigned char*>(a + t * term_stride + off),
+                      S::kOpBytes, fb);
+            bulk_load(base + (kTerms + t) * S::kOpBytes,
+                      reinterpret_cast<const unsigned char*>(b + t * term_stride + off), S::kOpBytes, fb);
           }
         }
+      }
+      if (!ok) {  // the copies in flight land before the CTA gives up its memory
+        const unsigned long long t0 = globaltimer_ns();
+        for (int k = max(0, item - S::kStages); k < item; ++k)
+          while (!mbar_try(smem_u32(&full[k % S::kStages]), static_cast<uint32_t>((k / S::kStages) & 1)) &&
+                 globaltimer_ns() - t0 < timeout_ns) {
+          }
       }
     }
-  } else if (warp == kUWarps - 1) {
-    // ---- MMA issue (one thread)
-    if (lane == 0) {
-      long long item = 0;
-      long long committed = -1;  // last stage commit
-      int acc_commits = 0;       // accumulator commits issued
-      for (int m = 0; m < my_tiles && ok; ++m) {
-        const int b = m & 1, v = m >> 1;
-        if (v >= 1 && !mbar_wait(smem_u32(&accempty[b]), static_cast<uint32_t>((v - 1) & 1), U.st, timeout_ns)) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem + static_cast<uint32_t>(b * kUN);
-        for (int ch = 0; ch < nchunks; ++ch, ++item) {
-          const int st = static_cast<int>(item % S::kStages);
-          if (!mbar_wait(smem_u32(&full[st]), static_cast<uint32_t>((item / S::kStages) & 1), U.st, timeout_ns)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sb = smem_u32(usm + st * S::kStageBytes);
-          for (int ia = kTerms - 1; ia >= 0; --ia)
-            for (int ib = kTerms - 1 - ia; ib >= 0; --ib) {
-              const uint32_t a0 = sb + ia * kUOpBytes, b0 = sb + (kTerms + ib) * kUOpBytes;
+  } else if (warp == kUEpi + 1) {
+    const bool one = elect_one();
+    int item = 0;
+    for (int m = 0; m < my_tiles && ok; ++m) {
+      const int b = m % kUAcc, use = m / kUAcc;
+      if (use >= 1 && !(ok = wait(&accempty[b], use - 1))) break;
+      const uint32_t acc = tmem + static_cast<uint32_t>(b * kUN);
+      for (int ch = 0; ch < nchunks; ++ch, ++item) {
+        const int st = item % S::kStages;
+        if (!(ok = wait(&full[st], item / S::kStages))) break;
+        const uint64_t a = umma_desc(smem_u32(usm) + static_cast<uint32_t>(st * S::kStageBytes), 256);
+        if (one) {
 #pragma unroll
-              for (int ks = 0; ks < kUK / 16; ++ks) {
-                const bool first = ch == 0 && ks == 0 && ia == kTerms - 1 && ib == kTerms - 1 - ia;
-                umma_bf16(acc, umma_desc(a0 + ks * 256, S::kRowGroup), umma_desc(b0 + ks * 256, S::kRowGroup),
-                          first ? 0u : 1u);
-              }
-            }
+          for (int ia = kTerms - 1; ia >= 0; --ia)
+#pragma unroll
+            for (int ib = kTerms - 1 - ia; ib >= 0; --ib)
+              umma_bf16(acc, a + ia * (S::kOpBytes >> 4), a + (kTerms + ib) * (S::kOpBytes >> 4),
+                        ch == 0 && ia == kTerms - 1 ? 0u : 1u);
           umma_commit(smem_u32(&empty[st]));
-          committed = item;
-        }
-        if (!ok) break;
-        umma_commit(smem_u32(&accfull[b]));
-        ++acc_commits;
-      }
-      if (!ok && committed >= 0) {
-        // let the MMAs already issued finish before the accumulators are released
-        const uint32_t mb = smem_u32(&empty[committed % S::kStages]);
-        const uint32_t par = static_cast<uint32_t>((committed / S::kStages) & 1);
-        const unsigned long long t0 = globaltimer_ns();
-        while (!mbar_try(mb, par) && globaltimer_ns() - t0 < timeout_ns) {
         }
       }
-      (void)acc_commits;
+      if (ok && one) umma_commit(smem_u32(&accfull[b]));
+    }
+    if (!ok) {  // MMAs already issued finish before the accumulators are released
+      if (one) umma_commit(smem_u32(idle));
+      const unsigned long long t0 = globaltimer_ns();
+      while (!mbar_try(smem_u32(idle), 0) && globaltimer_ns() - t0 < timeout_ns) {
+      }
     }
   } else {
-    // ---- epilogue
-    for (int m = 0; m < my_tiles && ok; ++m) {
-      const int b = m & 1, v = m >> 1;
-      int i0, j0;
-      tile_of(static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), i0, j0);
-      const int i = i0 + warp * 32 + lane;  // this thread's row of the tile
-      const bool row_ok = i >= e && i < U.n;
-      if (row_ok) {
-        const double* row = U.c + static_cast<long long>(i) * U.ldc;
-        for (int jc = max(j0, i) & ~15; jc < min(j0 + kUN, U.n); jc += 16)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(row + jc));
-      }
-      if (!mbar_wait(smem_u32(&accfull[b]), static_cast<uint32_t>(v & 1), U.st, timeout_ns)) {
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int is = min(max(i, split_i0), U.n - 1);  // scale block of a row inside the matrix
-      const double sa = U.a_scale[(is - split_i0) / kBM];
-      double* crow = U.c + static_cast<long long>(is) * U.ldc;
-      // C values of the 8-column group at c0 (entries this thread does not
-      // update read as 0); the next group's load is in flight while a group
-      // is updated
-      auto load_c = [&](int c0, double (&cv)[8]) {
-#pragma unroll
-        for (int u = 0; u < 8; u += 2) {
-          const int j = j0 + c0 + u;
-          const bool ok0 = row_ok && j >= e && j < U.n && i <= j;
-          const bool ok1 = row_ok && j + 1 >= e && j + 1 < U.n && i <= j + 1;
-          if (ok0 && ok1) {
-            const double2 t = *reinterpret_cast<const double2*>(crow + j);
-            cv[u] = t.x;
-            cv[u + 1] = t.y;
-          } else {
-            cv[u] = ok0 ? crow[j] : 0.0;
-            cv[u + 1] = ok1 ? crow[j + 1] : 0.0;
-          }
-        }
+    const int wr = (warp & 3) * 32, wc = (warp >> 2) * kUCols;  // this warp's part of a tile
+    for (int m = 0; m < my_tiles; ++m) {
+      const int b = m % kUAcc, use = m / kUAcc;
+      int I, J;
+      tile_of(m, I, J);
+      const int i0 = t_i0 + I * kUM, j0 = t_i0 + J * kUN + wc;
+      const int ir = i0 + wr + (lane >> 2), jc = j0 + 2 * (lane & 3);
+      // one scale block of 64 rows and one of 64 columns hold the whole part
+      const int is = min(max(i0 + wr, split_i0), U.n - 1), js = min(max(j0, split_i0), U.n - 1);
+      const double unscale = 1.0 / (U.a_scale[(is - split_i0) / kBM] * U.b_scale[(js - split_i0) / kBM]);
+      double* cp = U.c + static_cast<long long>(ir) * U.ldc + jc;
+      const long long step = 8 * U.ldc;
+      const bool inside = i0 >= e && i0 + kUM <= U.n && i0 + kUM <= j0 && j0 + kUCols <= U.n;
+      auto mine = [&](int q, int c) {  // row ir + 8 q, column jc + c of the trailing upper triangle
+        const int i = ir + 8 * q, j = jc + c;
+        return i >= e && i < U.n && j >= e && j < U.n && i <= j;
       };
-      double cur[8], nxt[8];
-      load_c(0, cur);
-      const uint32_t tacc = tmem + static_cast<uint32_t>(b * kUN) + (static_cast<uint32_t>(warp * 32) << 16);
-#pragma unroll 1
-      for (int c0 = 0; c0 < kUN; c0 += 8) {
-        uint32_t r[8];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                       "=r"(r[7])
-                     : "r"(tacc + static_cast<uint32_t>(c0)));
-        if (c0 + 8 < kUN) load_c(c0 + 8, nxt);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int jb = j0 + c0;
-        const int js = min(max(jb, split_i0), U.n - 1);
-        const double unscale = 1.0 / (sa * U.b_scale[(js - split_i0) / kBM]);
-        if (row_ok) {
+      // C as tmem_ld16x8 has the sums: v[h][g][.] holds rows 16 h .. 16 h +
+      // 15, columns 8 g .. 8 g + 7
+      double v[2][kUCols / 8][4];
 #pragma unroll
-          for (int u = 0; u < 8; u += 2) {
-            const int j = jb + u;
-            const double v0 = cur[u] - static_cast<double>(__uint_as_float(r[u])) * unscale;
-            const double v1 = cur[u + 1] - static_cast<double>(__uint_as_float(r[u + 1])) * unscale;
-            const bool ok0 = j >= e && j < U.n && i <= j;
-            const bool ok1 = j + 1 >= e && j + 1 < U.n && i <= j + 1;
-            if (ok0 && ok1) {
-              *reinterpret_cast<double2*>(crow + j) = make_double2(v0, v1);
-            } else {
-              if (ok0) crow[j] = v0;
-              if (ok1) crow[j + 1] = v1;
-            }
+      for (int g = 0; g < kUCols / 8; ++g)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          double* vv = &v[q >> 1][g][(q & 1) * 2];
+          const double* p = cp + q * step + 8 * g;
+          if (inside) {
+            const double2 c = *reinterpret_cast<const double2*>(p);
+            vv[0] = c.x;
+            vv[1] = c.y;
+          } else {
+            vv[0] = mine(q, 8 * g) ? p[0] : 0.0;
+            vv[1] = mine(q, 8 * g + 1) ? p[1] : 0.0;
           }
         }
+      if (!(ok = wait(&accfull[b], use))) break;
+      const uint32_t tacc = tmem + static_cast<uint32_t>(b * kUN + wc) + (static_cast<uint32_t>(wr) << 16);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) cur[u] = nxt[u];
-      }
-      // this warp is done reading the accumulator
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int g = 0; g < kUCols / 8; g += 2) {
+          int d[2][4];
+          tmem_ld16x8(tacc + (static_cast<uint32_t>(16 * h) << 16) + 8 * g, d[0]);
+          tmem_ld16x8(tacc + (static_cast<uint32_t>(16 * h) << 16) + 8 * g + 8, d[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            double& c = v[h][g + (x >> 2)][x & 3];
+            c = c - static_cast<double>(__int_as_float(d[x >> 2][x & 3])) * unscale;
+          }
+        }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&accempty[b]));
+#pragma unroll
+      for (int g = 0; g < kUCols / 8; ++g)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double* vv = &v[q >> 1][g][(q & 1) * 2];
+          double* p = cp + q * step + 8 * g;
+          if (inside) {
+            *reinterpret_cast<double2*>(p) = make_double2(vv[0], vv[1]);
+          } else {
+            if (mine(q, 8 * g)) p[0] = vv[0];
+            if (mine(q, 8 * g + 1)) p[1] = vv[1];
+          }
+        }
     }
   }
   if (!ok) {
@@ -1426,8 +1403,8 @@ __global__ void __launch_bounds__(kUBlock, 2) umma_bf16s_update_kernel(UpdArgs U
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == kUWarps - 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kUN) : "memory");
+  if (warp == kUEpi + 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kUAcc * kUN) : "memory");
 }
 
 template <int kTerms>
@@ -1446,7 +1423,7 @@ int launch_umma_bf16(const UpdArgs& U, const __nv_bfloat16* ah, const __nv_bfloa
   BBK_CUDA_TRY(attr_err);
   const long long tm = (order + kUM - 1) / kUM + 1;
   const long long tiles = tm * (tm + 1) / 2;
-  const int grid = static_cast<int>(std::max(1LL, std::min<long long>(tiles, 2LL * device_sm_count())));
+  const int grid = static_cast<int>(std::max(1LL, std::min<long long>(tiles, device_sm_count())));
   umma_bf16s_update_kernel<kTerms><<<grid, kUBlock, S::kBytes, s>>>(U, ah, bh, kpad, term_stride,
                                                                     wait_timeout_ns());
   BBK_CUDA_TRY(cudaGetLastError());

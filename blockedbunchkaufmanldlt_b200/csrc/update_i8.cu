@@ -51,7 +51,6 @@ constexpr int kThreads = (kEpiWarps + 2) * 32;
 constexpr size_t kSmem = static_cast<size_t>(kStages) * kStageBytes + kEpiWarps * kCols * sizeof(double) + 256;
 static_assert(kSmem <= 227 * 1024, "stages fit the shared memory of one CTA");
 
-constexpr int kStrip = 12;  // tile columns of a strip: 12 x 12 tiles for 148 CTAs
 constexpr int kMaxExp = 400;  // larger scales go to the FP64 kernel
 constexpr int kMaxK = 1024;   // keeps 5 x k x 2^14 x 2^24 below 2^51: the joined sums are exact doubles
 
@@ -297,27 +296,6 @@ __device__ __forceinline__ void chunk_products(uint32_t tmem, uint64_t a, uint64
   }
 }
 
-// One lane of the (converged) warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-  return p != 0;
-}
-
-__device__ __forceinline__ void bulk_load(uint32_t dst, const unsigned char* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-// 16 rows x 8 columns of an accumulator: v[0], v[1] row lane / 4, v[2], v[3]
-// row lane / 4 + 8, at columns 2 (lane % 4) and the next.
-__device__ __forceinline__ void tmem_ld16x8(uint32_t addr, int (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"(addr));
-}
-
 // An integer below 2^51 in magnitude as a double, exactly.
 __device__ __forceinline__ double int_to_double(long long v) {
   return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
@@ -374,28 +352,8 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  // tile m of this CTA: the upper triangle in strips of kStrip tile columns,
-  // row by row within a strip, so the CTAs that run together share a few row
-  // and column blocks of digits in L2
-  auto tile_of = [&](int m, int& I, int& J) {
-    const int t = static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x);
-    constexpr int kTri = kStrip * (kStrip + 1) / 2;
-    auto before = [](int q) { return kStrip * kStrip * (q * (q - 1) / 2) + kTri * q; };  // tiles of the strips < q
-    int q = static_cast<int>(sqrt(2.0 * t) / kStrip);
-    while (q > 0 && before(q) > t) --q;
-    while (before(q + 1) <= t) ++q;
-    const int j0 = q * kStrip, w = min(kStrip, tm - j0);
-    int u = t - before(q);
-    if (u < w * j0) {
-      I = u / w;
-      J = j0 + u % w;
-      return;
-    }
-    u -= w * j0;
-    int j = 0;
-    while ((j + 1) * (j + 2) / 2 <= u) ++j;
-    I = j0 + u - j * (j + 1) / 2;
-    J = j0 + j;
+  auto tile_of = [&](int m, int& I, int& J) {  // tile m of this CTA
+    strip_tile(static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), tm, I, J);
   };
   const size_t row_block = static_cast<size_t>(S.nkc) * (kDigits * kBlock);
   bool ok = true;
