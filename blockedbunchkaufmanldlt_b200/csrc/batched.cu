@@ -34,8 +34,10 @@
 // trailing update in FP32 and refines the solution in FP64.
 #include <algorithm>
 #include <climits>
+#include <functional>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "bbk_internal.cuh"
@@ -1055,14 +1057,45 @@ const void* batched_kernel_of(int mode) {
                                          : reinterpret_cast<const void*>(batched_kernel<BBK_UPDATE_FP32, kC>);
 }
 
+// Whether a batch (largest first) finishes sooner with two CTAs per SM.  An
+// SM does up to twice the work with two, but each matrix takes longer: order
+// 512 2.6 -> 3.6 ms, 256 0.69 -> 0.85, 128 0.33 -> 0.35.  With few matrices of
+// mixed orders the largest one is the batch's time, and it should have its SM
+// to itself (220 of order 64..512: 3.26 ms with two CTAs, 2.52 with one; 400:
+// 3.49 and 2.90).  So both are estimated by giving each matrix in
+// turn to the CTA that is free first, in units of one pivot step (2 us): an
+// order n alone takes n steps and 640 (n / 512)^3 for its updates, with a
+// neighbour 1.05 + 0.35 n / 512 times that.
+bool pairs_finish_sooner(const std::vector<BatchItemDev>& v, int sms) {
+  if (v.size() >= 32 * static_cast<size_t>(sms)) return true;  // the queue evens out
+  auto finish = [&](int ctas, bool shared) {
+    std::priority_queue<float, std::vector<float>, std::greater<float>> free_at;
+    float end = 0.0f;
+    for (const BatchItemDev& it : v) {
+      const float x = it.n / 512.0f;
+      float t = it.n + 640.0f * x * x * x;
+      if (shared) t *= 1.05f + 0.35f * x;
+      if (static_cast<int>(free_at.size()) == ctas) {
+        t += free_at.top();
+        free_at.pop();
+      }
+      free_at.push(t);
+      end = std::max(end, t);
+    }
+    return end;
+  };
+  return finish(2 * sms, true) < finish(sms, false);
+}
+
 constexpr size_t kHeaderBytes = 256;
 
 // Host-side record of planned workspaces, so a launch needs no device read:
-// the largest order, and the most shared memory an item takes, with one CTA
-// per SM and with two.
+// the largest order, the most shared memory an item takes, with one CTA per
+// SM and with two, and whether two CTAs per SM finish the batch sooner.
 struct BatchPlanInfo {
   int count, max_n;
   size_t smem, smem_half;
+  bool pairs;
 };
 std::mutex g_plan_mu;
 std::map<const void*, BatchPlanInfo> g_plans;
@@ -1172,7 +1205,7 @@ extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const in
   BBK_CUDA_TRY(cudaMemcpyAsync(L.items, v.data(), v.size() * sizeof(BatchItemDev), cudaMemcpyHostToDevice, s));
   BBK_CUDA_TRY(cudaStreamSynchronize(s));
   // the launch reads these back without a device round trip
-  batch_plan_record(workspace, BatchPlanInfo{count, max_n, smem, smem_half});
+  batch_plan_record(workspace, BatchPlanInfo{count, max_n, smem, smem_half, pairs_finish_sooner(v, grid)});
   return BBK_OK;
 }
 
@@ -1195,13 +1228,14 @@ extern "C" int bbk_batched_factor_solve(int count, double* a, const double* a_or
   BatchLayout L = batch_layout(workspace, count, max_n, grid);
   if (workspace_bytes < L.bytes)
     return set_error(BBK_ERR_WORKSPACE, "batched workspace of %zu bytes, %zu needed", workspace_bytes, L.bytes);
-  // Two CTAs per SM where every item fits half of its shared memory (FP64:
-  // in the lean layout if need be) and the workspace has scratch for them.
+  // Two CTAs per SM where the batch gains by them, every item fits half of its
+  // shared memory (FP64: in the lean layout if need be) and the workspace has
+  // scratch for them.
   const size_t two = batch_layout(nullptr, count, max_n, 2 * grid).bytes;
   const bool lean =
       update_mode == BBK_UPDATE_FP64 && plan.smem > kHalfSmem && plan.smem_half <= kHalfSmem && workspace_bytes >= two;
   const size_t smem = lean ? plan.smem_half : plan.smem;
-  if (smem <= kHalfSmem && workspace_bytes >= two) grid *= 2;
+  if (plan.pairs && smem <= kHalfSmem && workspace_bytes >= two) grid *= 2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BatchArgs B{};
   B.count = count;

@@ -46,6 +46,24 @@ def test_two_ctas_per_sm_pivot_like_the_oracle(cuda, bbk, port, sizes, blocks):
     _check(port, plan, mats, rhs, x, perm, pt)
 
 
+@pytest.mark.parametrize("sizes", [
+    [16 + k % 25 for k in range(300)],             # two CTAs per SM finish sooner
+    [256, 200, 192] + [16] * 200,                  # the largest would hold the others up
+])
+def test_one_or_two_ctas_per_sm_give_the_same_bits(cuda, bbk, sizes):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def one(plan):
+        moved, n = 132, max(sizes)
+        stride = -(-(2 * moved * n + 3 * n + 2 * moved * 66 + moved) // 32) * 32
+        return plan.bytes - sms * stride * ctypes.sizeof(ctypes.c_double)
+
+    got, want = _run(bbk, sizes), _run(bbk, sizes, bytes_of=one)
+    for g, w in zip(got[3:], want[3:]):
+        assert np.array_equal(g, w)
+
+
 def test_workspace_for_one_cta_per_sm_is_still_accepted(cuda, bbk, port):
     import torch
     sizes = [512, 300, 64, 17]
