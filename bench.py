@@ -48,6 +48,8 @@ METRIC = "LDL^T solve GFLOP/s: FP64 vs FP32/BF16+IR at <=1e-12 bwd err; batched 
 UNIT = "GFLOP/s"
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6650.0
+FALLBACK_BF16_TFLOPS = 1400.0
+DIGIT_PRODUCTS = 34  # INT8 products per FP64 product of the digit update (csrc/update_i8.cu)
 
 
 def parse_args():
@@ -282,6 +284,31 @@ def update_flops(n: int, panel_end) -> float:
     return f
 
 
+def digit_update_flops(n: int, blk: int, panel_end) -> float:
+    """The part of update_flops that the integer tensor cores do: the panels
+    whose trailing order and block size reach the line drawn in
+    csrc/update_i8.cu (launch_update_i8)."""
+    f, k0 = 0.0, 0
+    for e in panel_end:
+        kb, m = e - k0, n - e
+        if m >= 1024 and m * blk >= 512 * 1024:
+            f += 2.0 * kb * m * (m + 1) / 2.0
+        k0 = e
+    return f
+
+
+def measured_int8_tops():
+    """INT8 tensor peak: twice the measured sustained cuBLAS bf16 rate (the
+    tensor cores' INT8 rate is twice their bf16 rate, under the same power
+    limit)."""
+    try:
+        with open(MEASURED_PEAKS) as fh:
+            return 2.0 * float(json.load(fh)["bf16_tflops_sustained"]), \
+                "2 x MEASURED_PEAKS.json bf16_tflops_sustained (measured)"
+    except (OSError, KeyError, ValueError):
+        return 2.0 * FALLBACK_BF16_TFLOPS, "2 x fallback 1.4 PFLOP/s sustained bf16"
+
+
 def panel_bytes(n: int, panel_end) -> float:
     """Compulsory DRAM bytes of the panel launches: each panel of width w
     starting at row k0 reads its w x (n - k0) strip of the matrix and writes
@@ -422,7 +449,18 @@ def run_main(args):
             "bound": "tensor", "achieved": upd_flops / (prof["update"]["ms"] / 1e3) / 1e12, "unit": "TFLOP/s",
             "peak": dgemm, "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 tensor peak)",
             "ms": prof["update"]["ms"], "launches": prof["update"]["launches"]}
-        kernels["trailing_update"]["frac"] = kernels["trailing_update"]["achieved"] / dgemm
+        # In the FP64 mode large panels run as INT8 digit products on the
+        # integer tensor cores, whose peak is then the one that bounds them;
+        # the FP64 rate stays beside it.
+        digit_flops = digit_update_flops(n, blk, pe_h) * args.steps if args.mode == "fp64" else 0.0
+        upd = kernels["trailing_update"]
+        upd["fp64_tflops"] = upd["achieved"]
+        upd["fp64_of_dgemm"] = upd["achieved"] / dgemm
+        if digit_flops > 0.5 * upd_flops:
+            upd["achieved"] = DIGIT_PRODUCTS * digit_flops / (prof["update"]["ms"] / 1e3) / 1e12
+            upd["unit"] = "TOP/s (INT8)"
+            upd["peak"], upd["peak_source"] = measured_int8_tops()
+        upd["frac"] = upd["achieved"] / upd["peak"]
     if prof["panel"]["ms"] > 0:
         kernels["panel"] = {
             "bound": "hbm", "achieved": pan_bytes / (prof["panel"]["ms"] / 1e3) / 1e9, "unit": "GB/s",
@@ -451,10 +489,13 @@ def run_main(args):
         else:
             units = upd_flops
         traffic = per_unit * units / dk["launches"]
+    update_units = "2 * width * m(m+1)/2 flops per panel update (m trailing rows), summed over the launches"
+    if "INT8" in kernels.get("trailing_update", {}).get("unit", ""):
+        update_units += (f"; as {DIGIT_PRODUCTS} INT8 operations per flop on the panels the digit update takes "
+                         "(achieved), traffic per FP64 flop")
     roofline = {"kernel": dom, "bound": dk["bound"], "achieved": dk["achieved"], "peak": dk["peak"],
                 "unit": dk["unit"], "frac": dk["frac"], "traffic": traffic, "peak_source": dk["peak_source"],
-                "algorithmic_units": ("2 * width * m(m+1)/2 flops per panel update (m trailing rows), "
-                                      "summed over the launches" if dom == "trailing_update" else
+                "algorithmic_units": (update_units if dom == "trailing_update" else
                                       "24 bytes per panel-strip entry (width x trailing order)")}
     if "panel" in kernels:
         # The panel is a chain of pivot steps, each needing one grid-wide

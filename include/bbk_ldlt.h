@@ -52,8 +52,10 @@ typedef enum bbk_status {
  * in-panel dot products keep the reference's summation order only in
  * BBK_UPDATE_FP64_ORDERED (elsewhere they are reassociated FMA chains). */
 typedef enum bbk_update_mode {
-  BBK_UPDATE_FP64 = 0,         /* FP64 tensor cores (DMMA mma.sync f64) for the
-                                  trailing update */
+  BBK_UPDATE_FP64 = 0,         /* trailing update at FP64 accuracy: large panels
+                                  as exact sums of 8-bit digit products on the
+                                  integer tensor cores (55-bit operands), small
+                                  ones on the FP64 tensor cores */
   BBK_UPDATE_FP64_ORDERED = 1, /* FP64, reference summation order: bitwise
                                   identical to the reference */
   BBK_UPDATE_FP32 = 2,         /* operands rounded to FP32, FP32 accumulate,
@@ -329,7 +331,9 @@ int bbk_update_trailing_block(int rows, int cols, int inner_dim,
  * its right-hand side at x + items[k].rhs (overwritten by the solution), and
  * its perm / pivot_types at perm + items[k].piv / pivot_types +
  * items[k].piv.  Block sizes are chosen per size bucket (n <= 32, 64, 128,
- * 256, 512, 1024); the library clamps each to what shared memory holds.
+ * 256, 512, 1024); the library clamps each to what shared memory holds, and
+ * BBK_UPDATE_FP64 may run a matrix in panels narrower than that, so that two
+ * matrices share an SM (the same pivots; other roundings).
  * ------------------------------------------------------------------------- */
 #define BBK_BATCH_MAX_N 1024
 #define BBK_BATCH_BUCKETS 6
@@ -347,7 +351,8 @@ typedef struct bbk_batch_info {
   double backward_error; /* max|b - A x| / (||A||_inf ||x||_inf + ||b||_inf) (refined modes) */
 } bbk_batch_info;
 
-/* Bytes of workspace for `count` items whose largest order is max_n. */
+/* Bytes of workspace for `count` items whose largest order is max_n (scratch
+ * for two CTAs per SM; with room for one per SM only, one runs). */
 size_t bbk_batched_workspace_size(int count, int max_n);
 /* Set-up (host, synchronous on `stream`): sorts the items largest first,
  * picks each item's block size from block_sizes[bucket] (NULL or 0 entries:

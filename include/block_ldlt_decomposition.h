@@ -41,7 +41,7 @@ class BlockLdltDecomposition {
   const std::vector<int>& PivotTypes() const { return pivot_types_; }
 
   // Extensions.  Trailing-update arithmetic (a bbk_update_mode): the default
-  // BBK_UPDATE_FP64 uses FP64 tensor cores; BBK_UPDATE_FP64_ORDERED
+  // BBK_UPDATE_FP64 uses the tensor cores; BBK_UPDATE_FP64_ORDERED
   // reproduces the reference bit for bit.
   void SetUpdateMode(int update_mode) { update_mode_ = update_mode; }
   // Solves A x = b for nrhs right-hand sides stored one after another (each
