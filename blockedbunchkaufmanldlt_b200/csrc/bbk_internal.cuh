@@ -267,7 +267,8 @@ int launch_finalize(const FactorPlan& plan, int panel, cudaStream_t s);
 int launch_left_swaps(const FactorPlan& plan, cudaStream_t s);
 int launch_wrows(const FactorPlan& plan, int panel, cudaStream_t s);
 int launch_update(const FactorPlan& plan, int panel, cudaStream_t s);
-int launch_update_i8(const FactorPlan& plan, int panel, long long order, const int** gate, cudaStream_t s);
+int launch_update_i8(const FactorPlan& plan, int panel, long long order, const int** gate,
+                     const unsigned char** marks, cudaStream_t s);
 int launch_status_copy(const DeviceState* st, int* status_out, cudaStream_t s);
 int launch_probe_wait(int ctas, int nslots, int iters, unsigned long long timeout_ns,
                       DeviceState* st, unsigned long long* slots, unsigned long long* stats,

@@ -60,9 +60,18 @@ struct UpdArgs {
   // BF16 mode: per 64-block power-of-two scales of A rows and B columns
   const double* a_scale;
   const double* b_scale;
-  // panel mode: run only when this flag is set (null: always)
+  // panel mode: run only when this flag is set (null: always): 1 all tiles, 2
+  // those in the 128 x 128 tiles that `marks` marks
   const int* gate;
+  const unsigned char* marks;
 };
+
+// Whether the tile at (i0, j0) is this launch's to update, of a trailing
+// matrix that starts at row e (see launch_update_i8).
+__device__ __forceinline__ bool marked(const UpdArgs& U, int e, int i0, int j0) {
+  const int t0 = e / 128 * 128, I = (i0 - t0) / 128, J = (j0 - t0) / 128;
+  return __ldcg(U.marks + J * (J + 1) / 2 + I) != 0;
+}
 
 __device__ __forceinline__ void cp_async_8(double* smem_dst, const double* gsrc, bool valid) {
   const unsigned saddr = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
@@ -357,7 +366,16 @@ __global__ void __launch_bounds__(kThreadsMma) mma_update_kernel(UpdArgs U) {
   extern __shared__ double smem[];
   if (!resolve_range(U)) return;
   const int ntiles = tile_count(U);
-  int t = blockIdx.x;
+  const bool some = U.gate != nullptr && ldcg(U.gate) == 2;
+  auto next = [&](int t) {  // this CTA's first tile from t on
+    for (; some && t < ntiles; t += gridDim.x) {
+      int I, J;
+      tile_coords(U, t, I, J);
+      if (marked(U, U.i_lo, U.tile_i0 + I * kBM, U.tile_j0 + J * kBN)) break;
+    }
+    return t;
+  };
+  int t = next(blockIdx.x);
   if (t >= ntiles) return;
   const int nchunks = (U.inner + kBK - 1) / kBK;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -407,7 +425,7 @@ __global__ void __launch_bounds__(kThreadsMma) mma_update_kernel(UpdArgs U) {
       if (ch + 1 < nchunks) cur = nxt;
     }
     // stage[cur] is free; stage[cur ^ 1] holds the C tile (vector path)
-    const int tn = t + static_cast<int>(gridDim.x);
+    const int tn = next(t + static_cast<int>(gridDim.x));
     int ni0 = 0, nj0 = 0;
     if (tn < ntiles) {
       int nI, nJ;
@@ -552,19 +570,24 @@ __global__ void __launch_bounds__(Wide<BM, BN, WM, WN, Stages, BK, MinBlocks>::k
   // (tile, chunk) items of this CTA, in order: tiles blockIdx.x + m * gridDim.x
   const int my_tiles = (ntiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                        static_cast<int>(gridDim.x);
-  const long long items = static_cast<long long>(my_tiles) * nchunks;
+  const bool some = U.gate != nullptr && ldcg(U.gate) == 2;
+  auto next = [&](int m, int& i0, int& j0) {  // this CTA's first tile from its m-th on, and its origin
+    for (; m < my_tiles; ++m) {
+      W::origin(U, static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), i0, j0);
+      if (!some || marked(U, U.i_lo, i0, j0)) break;
+    }
+    return m;
+  };
   long long ld_item = 0;  // loader cursor: item ld_item = tile ld_m, chunk ld_ch
-  int ld_ch = 0, ld_m = 0, ld_i0 = 0, ld_j0 = 0;
-  W::origin(U, blockIdx.x, ld_i0, ld_j0);
+  int ld_ch = 0, ld_i0 = 0, ld_j0 = 0;
+  int ld_m = next(0, ld_i0, ld_j0);
   auto issue = [&]() {
-    if (ld_item < items) {
+    if (ld_m < my_tiles) {
       W::load(U, smem + static_cast<size_t>(ld_item % Stages) * W::kStage, ld_i0, ld_j0, ld_ch * BK);
       ++ld_item;
       if (++ld_ch == nchunks) {
         ld_ch = 0;
-        ++ld_m;
-        if (ld_m < my_tiles)
-          W::origin(U, static_cast<int>(blockIdx.x) + ld_m * static_cast<int>(gridDim.x), ld_i0, ld_j0);
+        ld_m = next(ld_m + 1, ld_i0, ld_j0);
       }
     }
     cp_async_commit();  // one group per item slot, empty past the end
@@ -573,9 +596,8 @@ __global__ void __launch_bounds__(Wide<BM, BN, WM, WN, Stages, BK, MinBlocks>::k
   for (int s = 0; s < Stages - 1; ++s) issue();
 
   long long item = 0;
-  for (int m = 0; m < my_tiles; ++m) {
-    int i0, j0;
-    W::origin(U, static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), i0, j0);
+  int i0, j0;
+  for (int m = next(0, i0, j0); m < my_tiles; m = next(m + 1, i0, j0)) {
     // the C tile's rows go to L2 now; the epilogue reads them after the k loop
     for (int r = threadIdx.x / (BN / 16); r < BM; r += W::kThreads / (BN / 16)) {
       const int i = i0 + r;
@@ -1651,7 +1673,7 @@ int launch_update(const FactorPlan& plan, int panel, cudaStream_t s) {
   // the FP64 ones
   static const bool digits = getenv("BBK_UPDATE_TILE") == nullptr;
   if (plan.mode == BBK_UPDATE_FP64 && vec && digits) {
-    const int rc = launch_update_i8(plan, panel, plan.n - nominal_e, &U.gate, s);
+    const int rc = launch_update_i8(plan, panel, plan.n - nominal_e, &U.gate, &U.marks, s);
     if (rc) return rc;
   }
   if (plan.mode == BBK_UPDATE_FP64 && vec) {

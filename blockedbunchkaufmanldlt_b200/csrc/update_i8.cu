@@ -17,6 +17,22 @@
 // Factorization residuals: 9.2e-14 (FP64 tensor cores 1.14e-13) at n = 16000,
 // 7.4e-15 (8.9e-15) on a spectral matrix of order 4000.
 //
+// A row's digits are fixed-point: an entry far below the row's largest keeps
+// fewer bits than a double would, and a product of such entries is inaccurate
+// by itself, whatever it adds up to by norm.  With u and w the scaled
+// magnitudes, of K entries each, sum(u w) of an entry of C is off by at most
+// 2^-56 (sum(u) + sum(w)) for the operands' rounding and 5.1 K 2^-64 for the
+// products left out.  So a pass over the leading 7 bits of the magnitudes
+// (bound_kernel, one product for 34) bounds sum(u w) from below, and a tile
+// of C holding an entry whose error could exceed 16 x 2^-53 sum(u w)
+// is left to the FP64 tensor cores, whose own bound is K 2^-53 sum(u w) (a
+// panel with more than half of its tiles left so goes there whole).  Against
+// |L| |D| |L^T|, in units of 2^-53, n = 2304, block 256, two index sets at scales s
+// and 1 coupled by entries of size 1: digits alone 2.6, 45 and 4485 at s = 10^3,
+// 10^4 and 10^6; with the bound 1.3, 2.4 and 2.5, the same as the FP64 tensor cores alone.
+// The random, KKT and spectral matrices timed here need 5 to 15 of the 16, a
+// few tiles of a KKT matrix's first panel more.
+//
 // Scaling, all by powers of two: factor row k of W is divided by w_k, its
 // largest trailing entry, and column k of U multiplied by it, so a panel
 // whose pivots differ in scale keeps every product's leading bits; then each
@@ -25,11 +41,12 @@
 // FP64 tensor-core kernel, which is launched behind this one and returns
 // unless the flag is set.
 //
-// Measured (B200): update at n = 40000, block 256: 758 -> 309 ms per
-// factorization; n = 16000, block 256: 48.9 -> 22.0 ms; n = 10000, block
-// 128: 13.9 -> 10.4 ms.
+// Measured (B200): update at n = 40000, block 256: 758 -> 321 ms per
+// factorization (12 of them the bound); n = 16000, block 256: 48.9 -> 23.4 ms;
+// n = 10000, block 128: 13.9 -> 11.1 ms.
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <mutex>
 
 #include "bbk_internal.cuh"
@@ -48,7 +65,10 @@ constexpr int kStages = 3;
 constexpr int kEpiWarps = 16;
 constexpr int kCols = 4 * kTile / kEpiWarps;  // columns of an epilogue warp
 constexpr int kThreads = (kEpiWarps + 2) * 32;
-constexpr size_t kSmem = static_cast<size_t>(kStages) * kStageBytes + kEpiWarps * kCols * sizeof(double) + 256;
+constexpr int kMaxTiles = 4096;  // of one CTA
+constexpr int kAll = 1, kSome = 2;  // what a panel's flag leaves to the FP64 kernel
+constexpr size_t kSmem = static_cast<size_t>(kStages) * kStageBytes + kEpiWarps * kCols * sizeof(double) + 256 +
+                         kMaxTiles;
 static_assert(kSmem <= 227 * 1024, "stages fit the shared memory of one CTA");
 
 constexpr int kMaxExp = 400;  // larger scales go to the FP64 kernel
@@ -70,7 +90,13 @@ struct SliceArgs {
   double* sa;       // 2^(scale exponent) per row of U, from the 128-aligned origin
   double* sb;       // the same per column of W, times 2^-70
   unsigned long long* wmax;  // 2 x (nkc * kChunk): bits of w_k, by panel parity
-  int* flag;        // 2: the panel is left to the FP64 kernel, by parity
+  int* flag;        // by panel parity: kAll the panel, kSome its marked tiles are left to the FP64 kernel
+  unsigned char* ma;  // leading 7 bits of U's scaled magnitudes: block (row block, k chunk)
+  unsigned char* mb;  // W's
+  int* ta;          // per row of U and column of W: its part of the least 2^14 sum(u w)
+  int* tb;          // that the digits are accurate enough for (kNone: an empty row)
+  unsigned char* marks;  // per tile (J (J + 1) / 2 + I): left to the FP64 kernel
+  int* count;       // marked tiles, CTAs done (zero between launches)
   unsigned long long timeout_ns;
 };
 
@@ -137,13 +163,21 @@ __device__ __forceinline__ int row_exponent(double m) {
   return m > 0.0 ? x + (f > 0.996) : 0;
 }
 
+constexpr int kNone = -(1 << 29);
+
+// A row's part of that least sum: 2^14 times ((1 / 8) sum(u) + 5.1 K / 4096) /
+// 16, from sum(u), its largest entry's scale taken out.
+__device__ __forceinline__ int row_threshold(double sum, int k) {
+  return __double2int_ru(1024.0 * (0.125 * sum + 5.1 / 4096.0 * k));
+}
+
 // Digits of both operands.  One CTA takes 32 rows (columns of W): lane l row
 // l, warp w the k groups w, w + 8, ... of 16.  The rows are read twice (the
 // scale, then the digits; the second time from L1 or L2) and each thread
 // stores 16 bytes per digit, eight lanes to a 128-byte core matrix.
 __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
   extern __shared__ int kexp[];  // exponent of w_k
-  __shared__ double red[8][32];
+  __shared__ double red[8][32], rsum[8][32];
   __shared__ int bad;
   Range r;
   if (!panel_range_of(S, r)) return;
@@ -169,6 +203,8 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
   __syncthreads();
   const int rows = (S.n - r.t0 + kTile - 1) / kTile * kTile;
   const int groups = rows / 32;
+  const int ntiles = (rows / kTile) * (rows / kTile + 1) / 2;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < ntiles; i += gridDim.x * 256) S.marks[i] = 0;
   for (int job = blockIdx.x; job < 2 * groups; job += gridDim.x) {
     const bool is_u = job < groups;
     const int rr = (is_u ? job : job - groups) * 32 + lane;  // row from the tiles' origin
@@ -183,7 +219,7 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
                    : 0.0;
       }
     };
-    double m = 0.0;
+    double m = 0.0, sum = 0.0;
     bool fin = true;
     for (int g = warp; g < 2 * nchunks; g += 8) {
       double v[16];
@@ -194,32 +230,43 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
         const double s = fabs(v[i]) * pow2(is_u ? kx : -kx);
         fin = fin && s <= DBL_MAX;
         m = fmax(m, s);
+        sum += s;
       }
     }
     red[warp][lane] = m;
+    rsum[warp][lane] = sum;
     if (!fin) bad = 1;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i) m = fmax(m, red[i][lane]);
     const int ex = row_exponent(m);
     if (ex > kMaxExp || ex < -kMaxExp) bad = 1;
-    if (warp == 0) (is_u ? S.sa : S.sb)[rr] = pow2(is_u ? ex : ex - 70);
+    if (warp == 0) {
+      (is_u ? S.sa : S.sb)[rr] = pow2(is_u ? ex : ex - 70);
+      sum = 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum += rsum[i][lane];
+      (is_u ? S.ta : S.tb)[rr] = m > 0.0 ? row_threshold(sum * pow2(-ex), r.inner) : kNone;
+    }
     unsigned char* dst = (is_u ? S.da : S.db) + static_cast<size_t>(rr / kTile) * S.nkc * (kDigits * kBlock) +
                          (rr % kTile / 8) * 256 + (rr % 8) * 16;
+    unsigned char* mdst = (is_u ? S.ma : S.mb) + static_cast<size_t>(rr / kTile) * S.nkc * kBlock +
+                          (rr % kTile / 8) * 256 + (rr % 8) * 16;
     for (int g = warp; g < 2 * nchunks; g += 8) {
       double v[16];
       load(g, v);
-      uint32_t d[kDigits][4];
+      uint32_t d[kDigits][4], mag[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        uint32_t lo[4], hi[4];
+        uint32_t lo[4], hi[4], top[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int kx = kexp[g * 16 + 4 * q + i];
           // y = x + 128 in every lower byte: the bytes of y, less 128 each,
           // are the signed digits of x
-          const long long y =
-              __double2ll_rn(v[4 * q + i] * pow2(55 - ex + (is_u ? kx : -kx))) + 0x0000808080808080ll;
+          const long long x = __double2ll_rn(v[4 * q + i] * pow2(55 - ex + (is_u ? kx : -kx)));
+          const long long y = x + 0x0000808080808080ll;
+          top[i] = static_cast<uint32_t>(static_cast<unsigned long long>(x < 0 ? -x : x) >> 32);
           lo[i] = static_cast<uint32_t>(y) ^ 0x80808080u;
           hi[i] = static_cast<uint32_t>(static_cast<unsigned long long>(y) >> 32) ^ 0x00008080u;
         }
@@ -227,6 +274,7 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
           const uint32_t sel = static_cast<uint32_t>(byte | ((byte + 4) << 4));
           return __byte_perm(__byte_perm(v4[0], v4[1], sel), __byte_perm(v4[2], v4[3], sel), 0x5410);
         };
+        mag[q] = gather(top, 2);
         d[0][q] = gather(hi, 2);
         d[1][q] = gather(hi, 1);
         d[2][q] = gather(hi, 0);
@@ -239,28 +287,34 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs S) {
 #pragma unroll
       for (int t = 0; t < kDigits; ++t)
         *reinterpret_cast<uint4*>(blk + t * kBlock) = make_uint4(d[t][0], d[t][1], d[t][2], d[t][3]);
+      *reinterpret_cast<uint4*>(mdst + static_cast<size_t>(g / 2) * kBlock + (g & 1) * 128) =
+          make_uint4(mag[0], mag[1], mag[2], mag[3]);
     }
     __syncthreads();  // red is written again
   }
   __syncthreads();
-  if (threadIdx.x == 0 && bad) atomicExch(S.flag + (S.panel & 1), 1);
+  if (threadIdx.x == 0 && bad) atomicExch(S.flag + (S.panel & 1), kAll);
 }
 
 // Instruction descriptor of kind::i8: 32-bit integer accumulators, signed A
-// and B, both K-major, M = N = 128.
-constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTile >> 3) << 17) |
-                            (static_cast<uint32_t>(kTile >> 4) << 24);
+// and B, both K-major, M = 128, N = cols.
+__host__ __device__ constexpr uint32_t umma_i8_desc(int cols) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(cols >> 3) << 17) |
+         (static_cast<uint32_t>(kTile >> 4) << 24);
+}
+constexpr uint32_t kIdesc = umma_i8_desc(kTile);
 
 // One MMA.  Products that share their A digit keep it in the tensor core's
 // operand buffer (kUse: 0 fills it, 1 reads it, 2 reads it for the last
 // time, 3 does without): with A and B read from shared memory each time, an MMA of this size
 // takes all of its bandwidth and leaves none for the copies.
 template <int kUse>
-__device__ __forceinline__ void umma_i8(uint32_t d, uint64_t da, uint64_t db, bool accumulate) {
+__device__ __forceinline__ void umma_i8(uint32_t d, uint64_t da, uint64_t db, bool accumulate,
+                                        uint32_t idesc = kIdesc) {
 #define BBK_UMMA_I8(use)                                                                 \
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                         \
                "tcgen05.mma.cta_group::1.kind::i8" use " [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), \
-               "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate ? 1u : 0u))
+               "l"(da), "l"(db), "r"(idesc), "r"(accumulate ? 1u : 0u))
   if (kUse == 0) BBK_UMMA_I8(".collector::a::fill");
   if (kUse == 1) BBK_UMMA_I8(".collector::a::use");
   if (kUse == 2) BBK_UMMA_I8(".collector::a::lastuse");
@@ -296,6 +350,258 @@ __device__ __forceinline__ void chunk_products(uint32_t tmem, uint64_t a, uint64
   }
 }
 
+// Marks the tiles whose sums of magnitudes are too small for the digits (see
+// the top of this file).  Persistent CTAs over steps of a row block times a
+// strip of `cb` column blocks, each CTA a run of consecutive steps down the
+// strips: the strip's columns stay in shared memory, so only the row blocks
+// stream from L2 (with both operands streamed per tile the pass took 2.4 us per
+// tile and CTA, a seventh of the update).  Warps 0-15 compare the sums (warp
+// w: rows 32 (w % 4).., columns 32 (w / 4).. of each block), then one warp for
+// the bulk copies and one that issues the MMAs.
+constexpr int kGroup = 4;  // chunks of a stage of the ring of row blocks
+constexpr int kRingBytes = kGroup * kBlock;
+constexpr int kRingMax = 12;
+constexpr int kAcc = 2;    // accumulators of 2 kTile columns
+constexpr size_t kBoundData = 208 * 1024;  // the strips' columns, then the ring
+constexpr size_t kBoundSmem = kBoundData + kEpiWarps * 2 * 32 * sizeof(int) + 512;
+static_assert(kBoundSmem <= 227 * 1024 && (2 * kRingMax + 4 + 2 * kAcc) * 8 + 4 <= 512, "shared memory of one CTA");
+
+struct BoundShape {
+  int cb;    // column blocks of a strip
+  int nbuf;  // strips in shared memory
+  int ring;  // stages of row blocks
+};
+__host__ __device__ inline BoundShape bound_shape(int nkc) {
+  BoundShape b{2, 2, 0};
+  if (b.nbuf * b.cb * nkc * kBlock > 144 * 1024) b.nbuf = 1;
+  if (b.nbuf * b.cb * nkc * kBlock > 144 * 1024) b.cb = 1;
+  const int left = (static_cast<int>(kBoundData) - b.nbuf * b.cb * nkc * kBlock) / kRingBytes;
+  b.ring = left < kRingMax ? left : kRingMax;
+  return b;
+}
+static_assert(kBoundData >= kMaxK / kChunk * kBlock + 2 * kRingBytes, "the widest panel leaves a ring");
+
+__global__ void __launch_bounds__(kThreads, 1) bound_kernel(SliceArgs S) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  int* cols = reinterpret_cast<int*>(sm + kBoundData);  // 2 x 32 columns' parts per epilogue warp
+  uint64_t* full = reinterpret_cast<uint64_t*>(cols + kEpiWarps * 64);
+  uint64_t* empty = full + kRingMax;
+  uint64_t* bfull = empty + kRingMax;
+  uint64_t* bempty = bfull + 2;
+  uint64_t* accfull = bempty + 2;
+  uint64_t* accempty = accfull + kAcc;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + kAcc);
+  Range r;
+  if (!panel_range_of(S, r)) return;
+  int* flag = S.flag + (S.panel & 1);
+  // (another CTA may raise it to kSome meanwhile; kAll was set before this kernel)
+  if (ldcg(flag) == kAll) return;
+  const BoundShape shape = bound_shape(S.nkc);
+  const int cb = shape.cb;
+  const int tm = (S.n - r.t0 + kTile - 1) / kTile;
+  // strip j: row blocks 0 .. min(cb (j + 1), tm) - 1, after cb j (j + 1) / 2
+  // steps of the strips before it
+  const int strips = (tm + cb - 1) / cb;
+  const int total = cb * strips * (strips - 1) / 2 + tm;
+  const int first = static_cast<int>(static_cast<long long>(total) * blockIdx.x / gridDim.x);
+  const int last = static_cast<int>(static_cast<long long>(total) * (blockIdx.x + 1) / gridDim.x);
+  if (first >= last) return;
+  int j0 = static_cast<int>((sqrtf(8.0f * first / cb + 1.0f) - 1.0f) * 0.5f);
+  while (j0 > 0 && cb * j0 * (j0 + 1) / 2 > first) --j0;
+  while (j0 + 1 < strips && cb * (j0 + 1) * (j0 + 2) / 2 <= first) ++j0;
+  const int i0 = first - cb * j0 * (j0 + 1) / 2;
+  const int nchunks = (r.inner + kChunk - 1) / kChunk;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+
+  if (warp == kEpiWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(kAcc * 2 * kTile)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (lane == 0) {
+      for (int b = 0; b < 2 * kRingMax + 4; ++b)  // full, empty, bfull, bempty
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[b])) : "memory");
+      for (int b = 0; b < kAcc; ++b) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&accfull[b])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&accempty[b])), "r"(kEpiWarps)
+                     : "memory");
+      }
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  auto wait = [&](uint64_t* bar, int phase) {  // of a whole warp
+    const bool got = mbar_wait(smem_u32(bar), static_cast<uint32_t>(phase & 1), S.st, S.timeout_ns);
+    if (!__all_sync(0xffffffffu, got)) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return true;
+  };
+  auto finish = [&](uint64_t* bar, int phase, unsigned long long t0) {  // whatever it is that still runs
+    while (!mbar_try(smem_u32(bar), static_cast<uint32_t>(phase & 1)) && globaltimer_ns() - t0 < S.timeout_ns) {
+    }
+  };
+  const size_t row_block = static_cast<size_t>(S.nkc) * kBlock;
+  const int strip_bytes = cb * S.nkc * kBlock;
+  const uint32_t ring0 = smem_u32(sm) + static_cast<uint32_t>(shape.nbuf * strip_bytes);
+  // the steps of this CTA, in order: f(step, strip's count here, row block,
+  // strip, first step of the strip, last step of it)
+  auto steps = [&](auto&& f) {
+    int i = i0, j = j0, strip = 0;
+    bool fresh = true;
+    for (int t = first; t < last; ++t) {
+      const bool ends = i + 1 == min(cb * (j + 1), tm) || t + 1 == last;
+      if (!f(t - first, strip, i, j, fresh, ends)) return false;
+      fresh = ends;
+      if (ends) {
+        i = 0;
+        ++j;
+        ++strip;
+      } else {
+        ++i;
+      }
+    }
+    return true;
+  };
+  bool ok = true;
+
+  if (warp == kEpiWarps) {
+    if (lane == 0) {
+      int item = 0, loaded = 0;
+      ok = steps([&](int, int strip, int i, int j, bool fresh, bool) {
+        if (fresh) {
+          const int b = strip % shape.nbuf, use = strip / shape.nbuf;
+          if (use >= 1 && !mbar_wait(smem_u32(&bempty[b]), static_cast<uint32_t>((use - 1) & 1), S.st, S.timeout_ns))
+            return false;
+          const int blocks = min(cb, tm - cb * j);
+          const uint32_t bar = smem_u32(&bfull[b]);
+          const uint32_t base = smem_u32(sm) + static_cast<uint32_t>(b * strip_bytes);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                       "r"(blocks * nchunks * kBlock)
+                       : "memory");
+          for (int ch = 0; ch < nchunks; ++ch)
+            for (int h = 0; h < blocks; ++h)
+              bulk_load(base + static_cast<uint32_t>((ch * cb + h) * kBlock),
+                        S.mb + (cb * j + h) * row_block + static_cast<size_t>(ch) * kBlock, kBlock, bar);
+          ++loaded;
+        }
+        for (int ch = 0; ch < nchunks; ch += kGroup, ++item) {
+          const int st = item % shape.ring;
+          if (item >= shape.ring && !mbar_wait(smem_u32(&empty[st]), static_cast<uint32_t>((item / shape.ring - 1) & 1),
+                                               S.st, S.timeout_ns))
+            return false;
+          const uint32_t bar = smem_u32(&full[st]);
+          const uint32_t bytes = static_cast<uint32_t>(min(kGroup, nchunks - ch) * kBlock);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+          bulk_load(ring0 + static_cast<uint32_t>(st * kRingBytes), S.ma + i * row_block + static_cast<size_t>(ch) * kBlock,
+                    bytes, bar);
+        }
+        return true;
+      });
+      // the copies in flight land before the CTA gives up its memory
+      const unsigned long long t0 = globaltimer_ns();
+      for (int k = max(0, item - shape.ring); k < item; ++k) finish(&full[k % shape.ring], k / shape.ring, t0);
+      for (int k = max(0, loaded - shape.nbuf); k < loaded; ++k) finish(&bfull[k % shape.nbuf], k / shape.nbuf, t0);
+    }
+  } else if (warp == kEpiWarps + 1) {
+    const bool one = elect_one();
+    int item = 0;
+    ok = steps([&](int step, int strip, int, int j, bool fresh, bool ends) {
+      const int b = strip % shape.nbuf, acc = step % kAcc;
+      if (fresh && !wait(&bfull[b], strip / shape.nbuf)) return false;
+      if (step >= kAcc && !wait(&accempty[acc], step / kAcc - 1)) return false;
+      const uint32_t idesc = umma_i8_desc(min(cb, tm - cb * j) * kTile);
+      const uint64_t bd = umma_desc(smem_u32(sm) + static_cast<uint32_t>(b * strip_bytes), 256);
+      for (int ch = 0; ch < nchunks; ch += kGroup, ++item) {
+        const int st = item % shape.ring;
+        if (!wait(&full[st], item / shape.ring)) return false;
+        const uint64_t ad = umma_desc(ring0 + static_cast<uint32_t>(st * kRingBytes), 256);
+        if (one) {
+          for (int c = 0; c < min(kGroup, nchunks - ch); ++c)
+            umma_i8<3>(tmem + static_cast<uint32_t>(acc * 2 * kTile), ad + c * (kBlock >> 4),
+                       bd + (ch + c) * cb * (kBlock >> 4), ch + c > 0, idesc);
+          umma_commit(smem_u32(&empty[st]));
+        }
+      }
+      if (one) {
+        umma_commit(smem_u32(&accfull[acc]));
+        if (ends) umma_commit(smem_u32(&bempty[b]));
+      }
+      return true;
+    });
+    // the MMAs issued finish before the accumulators are released
+    if (item > 0) finish(&empty[(item - 1) % shape.ring], (item - 1) / shape.ring, globaltimer_ns());
+  } else {
+    const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 32;  // this thread's row, its columns
+    int* tb = cols + warp * 64;
+    int ta = S.ta[i0 * kTile + row];
+    ok = steps([&](int step, int, int i, int j, bool fresh, bool ends) {
+      const int acc = step % kAcc, blocks = min(cb, tm - cb * j);
+      if (fresh) {
+        __syncwarp();  // every lane is done with the last strip's columns
+        for (int h = 0; h < blocks; ++h) tb[h * 32 + lane] = S.tb[(cb * j + h) * kTile + col0 + lane];
+        __syncwarp();
+      }
+      const int t = ta;
+      if (step + 1 < last - first) ta = S.ta[(ends ? 0 : i + 1) * kTile + row];  // on its way during the wait
+      if (!wait(&accfull[acc], step / kAcc)) return false;
+      unsigned low = 0;  // bit h: an entry of block h
+      for (int h = 0; h < blocks; ++h) {
+        int p[32];
+        tmem_ld32x32(tmem + static_cast<uint32_t>(acc * 2 * kTile + h * kTile + col0) +
+                         (static_cast<uint32_t>((warp & 3) * 32) << 16), p);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int J = cb * j + h;
+        if (i > J) continue;
+        const int from = i == J ? row - col0 : 0;  // the upper triangle's columns of this row
+        int least = INT_MAX;
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          const int v = p[c] - tb[h * 32 + c];
+          least = min(least, c >= from ? v : INT_MAX);
+        }
+        if (least < t) low |= 1u << h;
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&accempty[acc]));
+      low = __reduce_or_sync(0xffffffffu, low);
+      if (low && lane == 0) {
+        for (int h = 0; h < blocks; ++h) {
+          const int J = cb * j + h;
+          const int tile = J * (J + 1) / 2 + i;
+          const unsigned bit = 1u << 8 * (tile & 3);
+          if ((low >> h & 1) && !(atomicOr(reinterpret_cast<unsigned*>(S.marks) + (tile >> 2), bit) & bit))
+            atomicAdd(S.count, 1);
+        }
+        atomicCAS(flag, 0, kSome);
+      }
+      return true;
+    });
+  }
+  if (!ok) {
+    atomicCAS(const_cast<int*>(&S.st->status), 0, BBK_ERR_TIMEOUT);
+    atomicExch(const_cast<int*>(&S.st->abort), 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == kEpiWarps + 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAcc * 2 * kTile)
+                 : "memory");
+  // the last CTA: beyond half of the tiles, the FP64 kernel takes all (a tile in
+  // digits takes 0.4 of its time there)
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(S.count + 1, 1) == min(total, static_cast<int>(gridDim.x)) - 1) {
+      if (2 * atomicExch(S.count, 0) > tm * (tm + 1) / 2) atomicExch(flag, kAll);
+      atomicExch(S.count + 1, 0);
+    }
+  }
+}
+
 // An integer below 2^51 in magnitude as a double, exactly.
 __device__ __forceinline__ double int_to_double(long long v) {
   return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
@@ -322,9 +628,11 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
   uint64_t* accfull = empty + kStages;
   uint64_t* accempty = accfull + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + 1);
+  unsigned char* skip = sm + kSmem - kMaxTiles;  // per tile of this CTA: left to the FP64 kernel
   Range r;
   if (!panel_range_of(S, r)) return;
-  if (ldcg(S.flag + (S.panel & 1))) return;
+  const int left = ldcg(S.flag + (S.panel & 1));  // what the FP64 kernel takes
+  if (left == kAll) return;
   const int tm = (S.n - r.t0 + kTile - 1) / kTile;
   const int ntiles = tm * (tm + 1) / 2;
   if (static_cast<int>(blockIdx.x) >= ntiles) return;
@@ -347,6 +655,11 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(accempty)), "r"(kEpiWarps) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+  }
+  for (int m = threadIdx.x; m < my_tiles; m += kThreads) {
+    int I, J;
+    strip_tile(static_cast<int>(blockIdx.x) + m * static_cast<int>(gridDim.x), tm, I, J);
+    skip[m] = left == kSome ? __ldcg(S.marks + J * (J + 1) / 2 + I) : 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -518,12 +831,13 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
           }
         }
       };
-      if (!(ok = wait_full(2 * m))) break;
+      if (!(ok = wait_full(0))) break;
       drain(1.0);
       release();
-      if (!(ok = wait_full(2 * m + 1))) break;
+      if (!(ok = wait_full(1))) break;
       drain(4294967296.0);
       release();
+      if (skip[m]) continue;
 #pragma unroll
       for (int g = 0; g < kCols / 8; ++g)
 #pragma unroll
@@ -553,9 +867,12 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
 }  // namespace
 
 // Launches the digit update of `panel` where it applies (see the rule below);
-// *gate is then the flag behind which the caller launches the FP64 kernel.
-int launch_update_i8(const FactorPlan& plan, int panel, long long order, const int** gate, cudaStream_t s) {
+// *gate and *marks then say what is left to the FP64 kernel that the caller
+// launches behind it (the flag: 0 nothing, 1 the panel, 2 the marked tiles).
+int launch_update_i8(const FactorPlan& plan, int panel, long long order, const int** gate,
+                     const unsigned char** marks, cudaStream_t s) {
   *gate = nullptr;
+  *marks = nullptr;
   // Sorting out digits and scales costs about 30 us per panel whatever the
   // width, and a tile's epilogue the same for any k, so the line lies at a
   // product of order and width (n = 8000, ms per factorization with the
@@ -564,16 +881,23 @@ int launch_update_i8(const FactorPlan& plan, int panel, long long order, const i
   // 7.72; block 64: 10.7 / 10.5 / 10.1 / 9.87 / 9.76).
   if (order * plan.b < 512 * 1024 || order < 1024) return BBK_OK;
   const long long npad = plan.ldw;
-  const size_t digits = static_cast<size_t>(kDigits) * npad * plan.kpad;
+  const size_t mags = static_cast<size_t>(npad) * plan.kpad;
+  const size_t digits = kDigits * mags;
+  const size_t tiles = static_cast<size_t>(npad / kTile + 1) * (npad / kTile + 2) / 2;
   // the digits live in what the update phase leaves idle of the workspace:
-  // U's in the BF16 operands' buffer, with the scales behind them, W's in
+  // U's in the BF16 operands' buffer, with the scales and marks behind them, W's in
   // the panel kernel's slot-ordered U and W (one after the other)
   char* hs = static_cast<char*>(plan.hsplit);
   char* us = reinterpret_cast<char*>(plan.uslot);
   const size_t us_room = static_cast<size_t>(reinterpret_cast<char*>(plan.wslot) - us) +
                          static_cast<size_t>(plan.b + 2) * npad * sizeof(double);
-  const size_t hs_need = digits + 2 * npad * sizeof(double) + (2 * plan.kpad + 2) * sizeof(unsigned long long);
-  if (plan.kpad > kMaxK || digits > us_room || hs_need > 12 * plan.hstride ||
+  const size_t hs_need = digits + mags + 2 * npad * sizeof(double) + (2 * plan.kpad + 2) * sizeof(unsigned long long) +
+                         2 * npad * sizeof(int) + tiles;
+  const int sms = device_sm_count();
+  const long long tm = order / kTile + 2;
+  const int grid = static_cast<int>(std::min<long long>(tm * (tm + 1) / 2, sms));
+  if (tm * (tm + 1) / 2 > static_cast<long long>(kMaxTiles) * grid) return BBK_OK;
+  if (plan.kpad > kMaxK || digits + mags > us_room || hs_need > 12 * plan.hstride ||
       reinterpret_cast<uintptr_t>(hs) % 16 || reinterpret_cast<uintptr_t>(us) % 16)
     return BBK_OK;
   SliceArgs S{};
@@ -589,10 +913,16 @@ int launch_update_i8(const FactorPlan& plan, int panel, long long order, const i
   S.nkc = plan.kpad / kChunk;
   S.da = reinterpret_cast<unsigned char*>(hs);
   S.db = reinterpret_cast<unsigned char*>(us);
-  S.sa = reinterpret_cast<double*>(hs + digits);
+  S.ma = S.da + digits;
+  S.mb = S.db + digits;
+  S.sa = reinterpret_cast<double*>(hs + digits + mags);
   S.sb = S.sa + npad;
   S.wmax = reinterpret_cast<unsigned long long*>(S.sb + npad);
   S.flag = reinterpret_cast<int*>(S.wmax + 2 * plan.kpad);
+  S.count = S.flag + 2;
+  S.ta = S.flag + 4;
+  S.tb = S.ta + npad;
+  S.marks = reinterpret_cast<unsigned char*>(S.tb + npad);
   S.timeout_ns = wait_timeout_ns();
   if (panel == 0)
     BBK_CUDA_TRY(cudaMemsetAsync(S.wmax, 0, (2 * plan.kpad + 2) * sizeof(unsigned long long), s));
@@ -604,21 +934,24 @@ int launch_update_i8(const FactorPlan& plan, int panel, long long order, const i
   std::call_once(attr_once[dev], [&] {
     attr_err = cudaFuncSetAttribute(i8_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(kSmem));
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(bound_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kBoundSmem));
   });
   BBK_CUDA_TRY(attr_err);
-  const int sms = device_sm_count();
   const int segs = static_cast<int>(std::max(1LL, std::min(16LL, order / 2048)));
   row_max_kernel<<<dim3(segs, plan.b + 1), 256, 0, s>>>(S);
   BBK_CUDA_TRY(cudaGetLastError());
   const int slices = static_cast<int>(std::min<long long>(4 * sms, 2 * ((order + 256) / 32)));
   slice_kernel<<<slices, 256, plan.kpad * sizeof(int), s>>>(S);
   BBK_CUDA_TRY(cudaGetLastError());
-  const long long tm = order / kTile + 2;
-  const int grid = static_cast<int>(std::min<long long>(tm * (tm + 1) / 2, sms));
+  bound_kernel<<<grid, kThreads, kBoundSmem, s>>>(S);
+  BBK_CUDA_TRY(cudaGetLastError());
   i8_update_kernel<<<grid, kThreads, kSmem, s>>>(S);
   BBK_CUDA_TRY(cudaGetLastError());
-  count_launch(3);
+  count_launch(4);
   *gate = S.flag + (panel & 1);
+  *marks = S.marks;
   return BBK_OK;
 }
 

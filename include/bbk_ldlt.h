@@ -54,8 +54,10 @@ typedef enum bbk_status {
 typedef enum bbk_update_mode {
   BBK_UPDATE_FP64 = 0,         /* trailing update at FP64 accuracy: large panels
                                   as exact sums of 8-bit digit products on the
-                                  integer tensor cores (55-bit operands), small
-                                  ones on the FP64 tensor cores */
+                                  integer tensor cores (55-bit operands) where
+                                  that keeps an entry's error below 16 2^-53 times
+                                  its sum of magnitudes |U| |W|, the rest and
+                                  small panels on the FP64 tensor cores */
   BBK_UPDATE_FP64_ORDERED = 1, /* FP64, reference summation order: bitwise
                                   identical to the reference */
   BBK_UPDATE_FP32 = 2,         /* operands rounded to FP32, FP32 accumulate,
