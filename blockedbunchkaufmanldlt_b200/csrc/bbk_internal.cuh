@@ -273,6 +273,7 @@ int launch_status_copy(const DeviceState* st, int* status_out, cudaStream_t s);
 int launch_probe_wait(int ctas, int nslots, int iters, unsigned long long timeout_ns,
                       DeviceState* st, unsigned long long* slots, unsigned long long* stats,
                       cudaStream_t s);
+int launch_probe_cluster(int ctas, unsigned long long timeout_ns, DeviceState* st, cudaStream_t s);
 int launch_update_block(int rows, int cols, int inner, const double* left, int ls,
                         const double* ws, int wss, double* target, int ts, int mode,
                         cudaStream_t s);

@@ -445,14 +445,34 @@ __device__ __forceinline__ bool cluster_wait(const PanelArgs& P, uint32_t bar, u
   }
 }
 
-// After a wait ran out: lets stores in flight land, and no CTA leaves while
-// another may still write to it.
-__device__ __forceinline__ void cluster_abandon() {
-  __nanosleep(20000);
+// After a wait of exchange `seq` ran out, `cols` column transfers into the
+// panel: the CTA stays until the stores of the others have landed.  At the
+// barrier they have sent all that they ever will, but it does not wait for
+// their st.async, so what this CTA expects is waited for (1 ms at most: a CTA that gave
+// up earlier has not sent it).  A CTA that is one exchange ahead may have sent
+// more, which nothing here counts; it left before the barrier and lands within
+// microseconds, of which 200 are waited in any case.
+__device__ __noinline__ void cluster_abandon(ClusterShared& C, unsigned seq, int cols) {
   cluster_barrier();
+  const unsigned long long t0 = globaltimer_ns();
+  auto land = [&](unsigned long long* bar, unsigned phase) {
+    uint32_t done = 0;
+    while (!done && globaltimer_ns() - t0 < 1000000)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}\n"
+          : "=r"(done)
+          : "r"(smem_addr(bar)), "r"(phase & 1u)
+          : "memory");
+  };
+  land(&C.bar[seq & 1], seq >> 1);
+  for (int k = max(0, cols - 1); k <= cols; ++k) land(&C.col[k & 1], static_cast<unsigned>(k >> 1));
+  while (globaltimer_ns() - t0 < 200000) {
+  }
 }
 
-template <bool kTwo, typename OwnerOf>
+// kMissing: words to wait for that nobody sends (the bounded-wait probe)
+template <bool kTwo, int kMissing = 0, typename OwnerOf>
 __device__ __forceinline__ XResult cluster_exchange(const PanelArgs& P, int G, unsigned seq, Cand ca, Cand cb,
                                                     const double* pub_in, OwnerOf&& pub_owner, int npub, XShared& X,
                                                     ClusterShared& C) {
@@ -469,7 +489,7 @@ __device__ __forceinline__ XResult cluster_exchange(const PanelArgs& P, int G, u
   __syncthreads();
   const unsigned long long t_stat = P.stats ? globaltimer_ns() : 0;
   const uint32_t bar = smem_addr(&C.bar[par]);
-  if (t == kThreads) expect_bytes(bar, G * (kRec + npub) * 8);
+  if (t == kThreads) expect_bytes(bar, (G * (kRec + npub) + kMissing) * 8);
   bool ok = C.failed == 0;
   {
     // every warp forms the record and sends it to its share of the CTAs
@@ -924,7 +944,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
                              ? cluster_exchange<false>(P, G, seq - 1, best, no_cand(), s_pub, owner_of, 3, X, C)
                              : exchange<false>(P, seq, false, best, no_cand(), s_pub, owner_of, 3, X);
       if (!x1.ok) {
-        if (kCluster) cluster_abandon();
+        if (kCluster) cluster_abandon(C, seq - 1, cols);
         return;
       }
       omega = x1.a.v;
@@ -1204,7 +1224,7 @@ __global__ void __launch_bounds__(kBlock, 1) panel_kernel(PanelArgs P) {
                                             X, C)
                    : exchange<true>(P, seq, false, Cand{sig, 0, 0, 0.0}, nx_best, s_pub, owner_of, spec ? 9 : 4, X);
       if (!x2.ok) {
-        if (kCluster) cluster_abandon();
+        if (kCluster) cluster_abandon(C, seq - 1, cols);
         return;
       }
       const double sigma = x2.a.v;
@@ -1745,6 +1765,37 @@ __global__ void __launch_bounds__(kBlock) probe_kernel(PanelArgs P) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && P.stats) P.stats[0] = globaltimer_ns() - t0;
 }
 
+// The cluster's bounded wait: a few exchanges, then one that also waits for
+// a word that nobody sends.
+__global__ void __launch_bounds__(kBlock) cluster_probe_kernel(PanelArgs P) {
+  __shared__ XShared X;
+  __shared__ double s_pub[kMaxPub];
+  __shared__ ClusterShared C;
+  if (threadIdx.x < kMaxPub) s_pub[threadIdx.x] = 0.0;
+  if (threadIdx.x == 0) {
+    C.failed = 0;
+    for (int k = 0; k < 2; ++k) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&C.bar[k])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&C.col[k])) : "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster_barrier();
+  const Cand mine{static_cast<double>(blockIdx.x), static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.x), 0.0};
+  auto owner = [](int) { return 0; };
+  unsigned seq = 0;
+  for (; seq < 5; ++seq)
+    if (!cluster_exchange<true>(P, gridDim.x, seq, mine, mine, s_pub, owner, 3, X, C).ok) {
+      cluster_abandon(C, seq, 0);
+      return;
+    }
+  if (!cluster_exchange<true, 1>(P, gridDim.x, seq, mine, mine, s_pub, owner, 3, X, C).ok) {
+    cluster_abandon(C, seq, 0);
+    return;
+  }
+  cluster_barrier();
+}
+
 }  // namespace
 
 static int cooperative_launch(const void* fn, int grid, PanelArgs* args, cudaStream_t s) {
@@ -2074,6 +2125,28 @@ int launch_probe_wait(int ctas, int nslots, int iters, unsigned long long timeou
   P.n = iters;
   P.stats = stats;
   return cooperative_launch(reinterpret_cast<const void*>(probe_kernel), ctas, &P, s);
+}
+
+int launch_probe_cluster(int ctas, unsigned long long timeout_ns, DeviceState* st, cudaStream_t s) {
+  PanelArgs P{};
+  P.st = st;
+  P.timeout_ns = timeout_ns;
+  int g = 1;
+  while (g < 8 && 2 * g <= ctas) g *= 2;  // 8: any device's clusters
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(g);
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = g;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  BBK_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_probe_kernel, P));
+  count_launch();
+  return BBK_OK;
 }
 
 }  // namespace bbk

@@ -82,7 +82,8 @@ unsigned long long bbk_kernel_launch_count(void);
 int bbk_set_wait_timeout_ns(unsigned long long timeout_ns);
 /* Test hook for the bounded-wait machinery: launches one cooperative grid of
  * `ctas` (1..223) blocks whose exchange also waits for one participant that
- * does not exist, so the wait must run out.  Returns BBK_ERR_TIMEOUT when the bound
+ * does not exist, so the wait must run out, and then one thread-block cluster
+ * (up to 8 blocks) likewise.  Returns BBK_ERR_TIMEOUT when the bound
  * works (and leaves the context usable), BBK_OK never. */
 int bbk_probe_bounded_wait(int ctas, unsigned long long timeout_ns, void* stream);
 /* Diagnostics: runs `iters` back-to-back grid exchanges (the panel kernel's

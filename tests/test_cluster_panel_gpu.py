@@ -61,8 +61,10 @@ def test_cluster_panels_with_degenerate_entries(cuda, bbk, port, value):
 
 def test_an_expired_wait_in_a_cluster_is_reported_and_the_context_survives(cuda, bbk):
     import torch
+    for ctas in (1, 2, 8):  # a grid's and a cluster's exchange that can never complete
+        assert bbk.probe_bounded_wait(ctas, 20_000_000) == bbk.BBK_ERR_TIMEOUT
     a = uniform_symmetric(900, 3)
-    bbk.set_wait_timeout_ns(1)
+    bbk.set_wait_timeout_ns(1)  # (whether a wait is this long is left to the device)
     try:
         try:
             bbk.factor_device(torch.from_numpy(a).to(cuda), 64)
