@@ -47,6 +47,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const 
   }
 }
 
+// Waits for phase `parity` of `mbar`, aborted or not, until a second after t0.
+// The copying and the MMA-issuing role of a tensor-memory kernel end with it,
+// whether they came to their end or gave up: what they issued is done before
+// the CTA gives up shared and tensor memory, also when only another role gave
+// up, and however short the caller's own wait limit is.
+__device__ __forceinline__ void mbar_finish(uint32_t mbar, uint32_t parity, unsigned long long t0) {
+  while (!mbar_try(mbar, parity) && globaltimer_ns() - t0 < 1000000000ull) {
+  }
+}
+
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }

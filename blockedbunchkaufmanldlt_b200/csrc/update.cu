@@ -1313,13 +1313,10 @@ __global__ void __launch_bounds__(kUBlock, 1) umma_bf16s_update_kernel(UpdArgs U
           }
         }
       }
-      if (!ok) {  // the copies in flight land before the CTA gives up its memory
-        const unsigned long long t0 = globaltimer_ns();
-        for (int k = max(0, item - S::kStages); k < item; ++k)
-          while (!mbar_try(smem_u32(&full[k % S::kStages]), static_cast<uint32_t>((k / S::kStages) & 1)) &&
-                 globaltimer_ns() - t0 < timeout_ns) {
-          }
-      }
+      // the copies in flight land before the CTA gives up its memory
+      const unsigned long long t0 = globaltimer_ns();
+      for (int k = max(0, item - S::kStages); k < item; ++k)
+        mbar_finish(smem_u32(&full[k % S::kStages]), static_cast<uint32_t>((k / S::kStages) & 1), t0);
     }
   } else if (warp == kUEpi + 1) {
     const bool one = elect_one();
@@ -1344,12 +1341,9 @@ __global__ void __launch_bounds__(kUBlock, 1) umma_bf16s_update_kernel(UpdArgs U
       }
       if (ok && one) umma_commit(smem_u32(&accfull[b]));
     }
-    if (!ok) {  // MMAs already issued finish before the accumulators are released
-      if (one) umma_commit(smem_u32(idle));
-      const unsigned long long t0 = globaltimer_ns();
-      while (!mbar_try(smem_u32(idle), 0) && globaltimer_ns() - t0 < timeout_ns) {
-      }
-    }
+    // the MMAs issued finish before the accumulators are released
+    if (one) umma_commit(smem_u32(idle));
+    mbar_finish(smem_u32(idle), 0, globaltimer_ns());
   } else {
     const int wr = (warp & 3) * 32, wc = (warp >> 2) * kUCols;  // this warp's part of a tile
     for (int m = 0; m < my_tiles; ++m) {

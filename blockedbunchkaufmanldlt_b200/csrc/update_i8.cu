@@ -439,9 +439,8 @@ __global__ void __launch_bounds__(kThreads, 1) bound_kernel(SliceArgs S) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     return true;
   };
-  auto finish = [&](uint64_t* bar, int phase, unsigned long long t0) {  // whatever it is that still runs
-    while (!mbar_try(smem_u32(bar), static_cast<uint32_t>(phase & 1)) && globaltimer_ns() - t0 < S.timeout_ns) {
-    }
+  auto finish = [&](uint64_t* bar, int phase, unsigned long long t0) {
+    mbar_finish(smem_u32(bar), static_cast<uint32_t>(phase & 1), t0);
   };
   const size_t row_block = static_cast<size_t>(S.nkc) * kBlock;
   const int strip_bytes = cb * S.nkc * kBlock;
@@ -697,13 +696,10 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
           bulk_load(base + bytes, b + off, bytes, bar);
         }
       }
-      if (!ok) {  // the copies in flight land before the CTA gives up its memory
-        const unsigned long long t0 = globaltimer_ns();
-        for (int k = max(0, item - kStages); k < item; ++k)
-          while (!mbar_try(smem_u32(&full[k % kStages]), static_cast<uint32_t>((k / kStages) & 1)) &&
-                 globaltimer_ns() - t0 < S.timeout_ns) {
-          }
-      }
+      // the copies in flight land before the CTA gives up its memory
+      const unsigned long long t0 = globaltimer_ns();
+      for (int k = max(0, item - kStages); k < item; ++k)
+        mbar_finish(smem_u32(&full[k % kStages]), static_cast<uint32_t>((k / kStages) & 1), t0);
     }
   } else if (warp == kEpiWarps + 1) {
     // the whole warp walks the stages, so that descriptors stay in uniform
@@ -746,13 +742,9 @@ __global__ void __launch_bounds__(kThreads, 1) i8_update_kernel(SliceArgs S) {
       if (!ok) break;
       if (one) umma_commit(smem_u32(accfull));
     }
-    if (!ok && committed >= 0) {  // MMAs already issued finish before the accumulators are released
-      const uint32_t mb = smem_u32(&empty[committed % kStages]);
-      const uint32_t par = static_cast<uint32_t>((committed / kStages) & 1);
-      const unsigned long long t0 = globaltimer_ns();
-      while (!mbar_try(mb, par) && globaltimer_ns() - t0 < S.timeout_ns) {
-      }
-    }
+    if (committed >= 0)  // the MMAs issued finish before the accumulators are released
+      mbar_finish(smem_u32(&empty[committed % kStages]), static_cast<uint32_t>((committed / kStages) & 1),
+                  globaltimer_ns());
   } else {
     const int half = (warp >> 2) * kCols;  // first column of this warp's part
     double* sb = scales + warp * kCols;
