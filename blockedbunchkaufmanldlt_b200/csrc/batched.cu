@@ -50,7 +50,10 @@ constexpr int kBWarps = kBT / 32;
 constexpr int kMaxB = 64;             // largest block size
 constexpr int kCap = 2 * kMaxB + 4;   // moved indices per panel
 constexpr int kWU = kMaxB + 2;        // a panel has at most b + 1 pivot rows
-constexpr size_t kBatchSmem = 220 * 1024;
+constexpr size_t kBatchSmem = 220 * 1024;  // bounds the block sizes (batch_block_bytes)
+// What a launch may ask for: the blocks that the bound lets through take up to
+// 230 688 bytes as they are laid out now (order 246, block 50).
+constexpr size_t kLaunchSmem = 226 * 1024;
 constexpr size_t kHalfSmem = 112 * 1024;  // two CTAs per SM
 constexpr int kSolveBlk = 32;
 
@@ -1183,7 +1186,7 @@ extern "C" int bbk_batched_plan(int count, const bbk_batch_item* items, const in
     int b = (block_sizes && block_sizes[bkt] > 0) ? block_sizes[bkt] : default_block(bkt);
     b = std::min(std::min(b, kMaxB), it.n);
     while (b > 1 && batch_block_bytes(it.n, b) > kBatchSmem) --b;
-    if (batch_block_bytes(it.n, b) > kBatchSmem)
+    if (batch_block_bytes(it.n, b) > kBatchSmem || batch_smem_bytes(it.n, b) > kLaunchSmem)
       return set_error(BBK_ERR_INVALID_ARGUMENT, "item %d: order %d does not fit shared memory", k, it.n);
     v[k] = BatchItemDev{it.n, it.lda, b, k, it.a, it.rhs, it.piv};
     if (chosen_blocks) chosen_blocks[k] = b;
@@ -1269,7 +1272,7 @@ extern "C" int bbk_batched_factor_solve(int count, double* a, const double* a_or
       for (int mode : {BBK_UPDATE_FP64_ORDERED, BBK_UPDATE_FP64, BBK_UPDATE_FP32})
         for (const void* k : {batched_kernel_of<1>(mode), batched_kernel_of<2>(mode), batched_kernel_of<4>(mode)})
           BBK_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(kBatchSmem)));
+                                            static_cast<int>(kLaunchSmem)));
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
