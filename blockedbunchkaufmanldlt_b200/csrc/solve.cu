@@ -12,11 +12,13 @@
 // published with a release flag.  The owner of a block gathers the
 // contributions of all earlier blocks into it, the old ones while the blocks
 // just before it are still being solved elsewhere, then solves its triangle
-// with inverses it formed meanwhile.  The critical path per block is one
-// flag, one fold and three 32 x 32 products.  Right-hand sides go in groups
-// of eight, up to sixteen groups side by side on CTAs of their own.
-// Measured: n = 10000, 1 right-hand side: 1.74 -> 1.34 ms (4.3 us per block);
-// n = 5000, 64: 11.4 -> 1.46 ms; n = 16000, 4: 3.07 -> 2.6 ms.
+// with inverses it formed meanwhile, or by substitution where they have grown.
+// The critical path per block is one flag, one fold and three 32 x 32 products.
+// Right-hand sides go in groups of eight, up to sixteen groups side by side on
+// CTAs of their own.
+// Measured: n = 10000, 1 right-hand side: 1.74 -> 1.38 ms (4.4 us per block,
+// 4.2 without the substitution's code behind the products); n = 5000, 64: 11.4 ->
+// 1.46 ms.  A block that is substituted through takes 2.7 us more.
 #include <algorithm>
 #include <mutex>
 
@@ -131,7 +133,7 @@ constexpr size_t kSweepSmem = (2 * kSB * kTriPitch + 4 * kMaxRhsChunk * kSB + kM
 // Each warp learns which blocks are solved on its own (one relaxed scan of
 // up to 32 flags, one acquire load of the newest set one, or a bounded wait
 // on the next), so no CTA barrier is taken per block.
-// Substitution through the triangle, one right-hand side per warp, took 2.7
+// Substitution through every triangle, one right-hand side per warp, took 2.7
 // of 5.5 us per block; the inverses are ready before the block's turn.
 __device__ __forceinline__ int ld_relaxed_flag(const int* p) {
   int v;
@@ -184,10 +186,21 @@ __device__ int warp_wait_solved(const SweepArgs& A, int k, int k_end, int fail) 
 // blocks by substitution, one column per thread, then the blocks below by
 // X21 = -X22 (L21 X11).  Only terms of the triangles enter (an infinity
 // times a zero beside them would not be a zero).  tmp: kInvTmp doubles.
-// Ends with a CTA barrier.
 // (The inverse of the whole triangle left residuals 6 to 15 % larger than
 // substitution does, n = 1000 and 2000; these leave the same.)
-__device__ void invert_unit_triangle(const double* tri, double* inv, double* tmp) {
+// Bunch-Kaufman does not bound L, and a product with an inverse is as accurate
+// as substitution only while the inverse does not grow.  So the inverse is not
+// used (*unusable is set) where an entry of it exceeds kGrowth times the largest
+// of 1 and its row's (backward: column's) entries of the triangle.  32 x 32
+// blocks with every entry below the diagonal c, largest backward error by
+// substitution / by the inverse, growth: c = -0.1: 1.3e-16 / 1.8e-16, 1.7; -0.12:
+// 1.1e-16 / 3.1e-16, 3.6; -0.15: 1.2e-16 / 7.5e-16, 9.9; -0.3: 9e-17 / 2.8e-14, 786;
+// -0.5: 8e-17 / 1.4e-12.  Blocks of Bunch-Kaufman factors of random, KKT and
+// spectral matrices: up to 4.3, 8 blocks of 1000 above 4.
+constexpr double kGrowth = 4.0;
+
+template <bool kForward>
+__device__ void invert_unit_triangle(const double* tri, double* inv, double* tmp, int* unusable) {
   constexpr int P = kTriPitch;
   const int t = threadIdx.x;
   for (int idx = t; idx < kSB * P; idx += kSolveThreads) inv[idx] = 0.0;
@@ -232,6 +245,18 @@ __device__ void invert_unit_triangle(const double* tri, double* inv, double* tmp
     }
   }
   __syncthreads();
+  // four threads per row (column) of its diagonal block
+  const int row = t >> 2, base = (row & ~31) + (t & 3) * 8;
+  auto at = [&](const double* m, int k) { return fabs(kForward ? m[(base + k) * P + row] : m[row * P + base + k]); };
+  double limit = 1.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) limit = fmax(limit, at(tri, k));
+  limit = fmax(limit, __shfl_xor_sync(0xffffffffu, limit, 1));
+  limit = kGrowth * fmax(limit, __shfl_xor_sync(0xffffffffu, limit, 2));
+  bool grown = false;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) grown = grown || !(at(inv, k) <= limit);
+  if (grown) *unusable = 1;
 }
 
 // The block's triangle, by halves h (backward: the transpose, the second half
@@ -239,19 +264,18 @@ __device__ void invert_unit_triangle(const double* tri, double* inv, double* tmp
 // Each product is 32 x 32: warp w takes the terms 4 w.. of row `lane`, the
 // eight partial sums are added by the thread of (right-hand side, row), which
 // returns its entries lane and lane + 32 of the solution.
-template <bool kForward, bool kMasked>
+template <bool kForward>
 __device__ __forceinline__ void solve_triangle(const double* tri, const double* inv, double* red, double* ys, int nc,
                                                double& x0, double& x1) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int cc0 = warp;
-  auto product = [&](bool masked, const double* m, int rows, int terms) -> double {
+  auto product = [&](const double* m, int rows, int terms) -> double {
     double acc[kMaxRhsChunk];
 #pragma unroll
     for (int cc = 0; cc < kMaxRhsChunk; ++cc) acc[cc] = 0.0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int k = 4 * warp + u;
-      if (masked && (kForward ? k > lane : k < lane)) continue;
       const double e = kForward ? m[(terms + k) * kTriPitch + rows + lane] : m[(rows + lane) * kTriPitch + terms + k];
 #pragma unroll
       for (int cc = 0; cc < kMaxRhsChunk; ++cc)
@@ -272,37 +296,46 @@ __device__ __forceinline__ void solve_triangle(const double* tri, const double* 
   };
   constexpr int g = kForward ? 0 : 32, h = 32 - g;
   double* yo = ys + cc0 * kSB;
-  const double xg = product(kMasked, inv, g, g);
+  const double xg = product(inv, g, g);
   __syncthreads();  // every term of r_g is read, and every partial sum
   if (cc0 < nc) yo[g + lane] = xg;
   __syncthreads();
-  const double th = product(false, tri, h, g);
+  const double th = product(tri, h, g);
   __syncthreads();
   if (cc0 < nc) yo[h + lane] -= th;
   __syncthreads();
-  const double xh = product(kMasked, inv, h, h);
+  const double xh = product(inv, h, h);
   x0 = kForward ? xg : xh;
   x1 = kForward ? xh : xg;
 }
 
-// The same from the right-hand sides r0, r1, terms outside the triangle left
-// out; the solution in ys.  (Out of line: it hardly ever runs.)
+// The same by substitution, a right-hand side per warp: its entries lane and
+// lane + 32 in x0, x1, the solution to y.  Terms outside the triangle and the
+// coupling entries of 2x2 pivots (types pt) do not enter.  (Where the inverse is
+// not used, and where a result is not finite.)
 template <bool kForward>
-__device__ __noinline__ void solve_triangle_masked(const double* tri, const double* inv, double* red, double* ys,
-                                                   int nc, double r0, double r1) {
-  const int lane = threadIdx.x & 31, cc0 = threadIdx.x >> 5;
-  if (cc0 < nc) {
-    ys[cc0 * kSB + lane] = r0;
-    ys[cc0 * kSB + 32 + lane] = r1;
+__device__ __forceinline__ void substitute(const double* tri, int bsz, const int* pt, double x0, double x1, double* y) {
+  const int i0 = threadIdx.x & 31, i1 = i0 + 32;
+  const unsigned lo = __ballot_sync(0xffffffffu, i0 < bsz && pt[i0] == 2);
+  const unsigned hi = __ballot_sync(0xffffffffu, i1 < bsz && pt[i1] == 2);
+  const unsigned long long open = static_cast<unsigned long long>(hi) << 32 | lo;  // bit k: a 2x2 starts at row k
+  if (kForward) {
+    for (int k = 0; k < bsz; ++k) {
+      const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
+      const int first = k + 1 + static_cast<int>(open >> k & 1);  // first row with a term of column k
+      if (i0 >= first) x0 = __fma_rn(-tri[k * kTriPitch + i0], xk, x0);
+      if (i1 >= first) x1 = __fma_rn(-tri[k * kTriPitch + i1], xk, x1);
+    }
+  } else {
+    for (int k = bsz - 1; k >= 0; --k) {
+      const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
+      const int last = k - 1 - static_cast<int>(k > 0 ? open >> (k - 1) & 1 : 0);
+      if (i0 <= last) x0 = __fma_rn(-tri[i0 * kTriPitch + k], xk, x0);
+      if (i1 <= last) x1 = __fma_rn(-tri[i1 * kTriPitch + k], xk, x1);
+    }
   }
-  __syncthreads();
-  double x0, x1;
-  solve_triangle<kForward, true>(tri, inv, red, ys, nc, x0, x1);
-  __syncthreads();
-  if (cc0 < nc) {
-    ys[cc0 * kSB + lane] = x0;
-    ys[cc0 * kSB + 32 + lane] = x1;
-  }
+  if (i0 < bsz) y[i0] = x0;
+  if (i1 < bsz) y[i1] = x1;
 }
 
 template <bool kForward>
@@ -312,7 +345,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
   double* inv = tri + kSB * kTriPitch;          // its inverse
   double* red = inv + kSB * kTriPitch;          // [4][kMaxRhsChunk][kSB] partial sums
   double* ys = red + 4 * kMaxRhsChunk * kSB;    // [kMaxRhsChunk][kSB]: the block being solved
-  __shared__ int s_fail;
+  __shared__ int s_fail, s_grown;
   const int n = A.n;
   const long long ldf = A.ldf;
   const int nblk = (n + kSB - 1) / kSB;
@@ -347,7 +380,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
     // the triangle's inverse, while earlier blocks are still being solved
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    invert_unit_triangle(tri, inv, red);
+    if (t == 0) s_grown = 0;
+    invert_unit_triangle<kForward>(tri, inv, red, &s_grown);
     // this block's right-hand sides, for the threads that finish them
     double yin[2];
 #pragma unroll
@@ -524,22 +558,21 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
     __syncthreads();
     // ---- the block's triangle.  The zeros beside a diagonal block's triangle
     // are harmless while everything is finite, and what is not shows in the
-    // result; then once more with the triangle's terms alone.
+    // result; then once more by substitution, as where the inverse has grown.
+    // (The products run either way, the flag waits in shared memory and the
+    // substitution is inline: with a branch around the products, a register for
+    // the flag or a call, n = 10000 took 1.40 to 1.47 ms.)
     const int cc0 = t >> 5;  // this thread's right-hand side
     double* yc = A.y + static_cast<long long>(cc0) * n + b0;
     const double r0 = cc0 < nc ? ys[cc0 * kSB + lane] : 0.0, r1 = cc0 < nc ? ys[cc0 * kSB + 32 + lane] : 0.0;
     double x0, x1;
-    solve_triangle<kForward, false>(tri, inv, red, ys, nc, x0, x1);
+    solve_triangle<kForward>(tri, inv, red, ys, nc, x0, x1);
     if (cc0 < nc) {
       if (lane < bsz) yc[lane] = x0;
       if (lane + 32 < bsz) yc[lane + 32] = x1;
     }
-    if (__syncthreads_or(!(isfinite(x0) && isfinite(x1)))) {
-      solve_triangle_masked<kForward>(tri, inv, red, ys, nc, r0, r1);
-      if (cc0 < nc) {
-        if (lane < bsz) yc[lane] = ys[cc0 * kSB + lane];
-        if (lane + 32 < bsz) yc[lane + 32] = ys[cc0 * kSB + 32 + lane];
-      }
+    if (__syncthreads_or(s_grown || !(isfinite(x0) && isfinite(x1)))) {
+      if (cc0 < nc) substitute<kForward>(tri, bsz, A.pt + b0, r0, r1, yc);
     }
     __syncthreads();
     if (t == 0) {
