@@ -18,7 +18,7 @@
 // CTAs of their own.
 // Measured: n = 10000, 1 right-hand side: 1.74 -> 1.38 ms (4.4 us per block,
 // 4.2 without the substitution's code behind the products); n = 5000, 64: 11.4 ->
-// 1.46 ms.  A block that is substituted through takes 2.7 us more.
+// 1.58 ms.  A block that is substituted through takes 2.7 us more.
 #include <algorithm>
 #include <mutex>
 
@@ -37,6 +37,16 @@ constexpr int kMaxRhsChunk = 8;   // right-hand sides of a group
 // 49 / 44 / 43; a sweep that reads the factor once for all of them: 11.4 and
 // 162).
 constexpr int kMaxGroups = 16;
+// Beyond this many right-hand sides the backward sweep sets the sums of every
+// kWindow blocks aside.  A lane's one running sum over all columns has an
+// error that grows with n: mean backward error of 64 right-hand sides, n = 2000,
+// 5000, 10000: 7.1e-16, 1.4e-15, 2.4e-15, with the sums set aside 6.8e-16, 1.0e-15,
+// 1.3e-15 (the sweep that read the factor once for all of them, and subtracted block
+// by block: 6.8e-16, 1.0e-15, 1.5e-15).  It takes 9 % longer (n = 5000, 64: 1.45 ->
+// 1.57 ms), with one right-hand side 15 %, so up to kPlainRhs, where the sums never were
+// split, they are not.
+constexpr int kPlainRhs = 32;
+constexpr int kWindow = 16;
 constexpr int kAhead = 4;         // factor blocks prefetched into L2 ahead of the fold
 
 __global__ void gather_kernel(int n, int nrhs, const double* b, long long ldb, const int* perm,
@@ -114,6 +124,8 @@ constexpr int kTriPitch = kSB + 1;
 constexpr int kInvTmp = 2 * 16 * 17;  // scratch of invert_unit_triangle, doubles
 static_assert(kInvTmp <= 4 * kMaxRhsChunk * kSB, "it fits the partial sums' space");
 constexpr size_t kSweepSmem = (2 * kSB * kTriPitch + 4 * kMaxRhsChunk * kSB + kMaxRhsChunk * kSB) * sizeof(double);
+constexpr size_t kAsideSmem = 8 * kMaxRhsChunk * kSolveThreads * sizeof(double);  // the sums set aside
+static_assert(kSweepSmem + kAsideSmem <= 227 * 1024, "they fit the shared memory of one CTA");
 
 // One sweep for up to kMaxGroups groups of kMaxRhsChunk right-hand sides, each
 // with CTAs and flags of its own.  CTA c of a group owns blocks c, c+G, ... in
@@ -338,13 +350,14 @@ __device__ __forceinline__ void substitute(const double* tri, int bsz, const int
   if (i1 < bsz) y[i1] = x1;
 }
 
-template <bool kForward>
+template <bool kForward, bool kAside>
 __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
   extern __shared__ double psm[];
   double* tri = psm;                            // [kSB][kTriPitch]: the block's triangle, by columns
   double* inv = tri + kSB * kTriPitch;          // its inverse
   double* red = inv + kSB * kTriPitch;          // [4][kMaxRhsChunk][kSB] partial sums
   double* ys = red + 4 * kMaxRhsChunk * kSB;    // [kMaxRhsChunk][kSB]: the block being solved
+  double* aside = ys + kMaxRhsChunk * kSB;      // [8][kMaxRhsChunk][kSolveThreads] (kAside)
   __shared__ int s_fail, s_grown;
   const int n = A.n;
   const long long ldf = A.ldf;
@@ -511,6 +524,24 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
               if (cc < nc) acc[j][cc] = __fma_rn(fc[j * 2 + h], yv[h][cc], acc[j][cc]);
 #pragma unroll
         for (int u = 0; u < 16; ++u) fc[u] = fn[u];
+        if (kAside && (k_first - k) % kWindow == kWindow - 1 && k > k_end) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int cc = 0; cc < kMaxRhsChunk; ++cc)
+              if (cc < nc) {
+                double* sum = aside + (j * kMaxRhsChunk + cc) * kSolveThreads + t;
+                *sum = k_first - k < kWindow ? acc[j][cc] : *sum + acc[j][cc];
+                acc[j][cc] = 0.0;
+              }
+        }
+      }
+      if (kAside && k_first - k_end >= kWindow) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int cc = 0; cc < kMaxRhsChunk; ++cc)
+            if (cc < nc) acc[j][cc] += aside[(j * kMaxRhsChunk + cc) * kSolveThreads + t];
       }
       // add the 64 sums of (j, cc) over the lanes by recursive halving: at
       // offset o each lane keeps one half of its values and adds the
@@ -707,19 +738,22 @@ int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const 
   if (dev < 0 || dev >= kMaxAttrDevices) return set_error(BBK_ERR_NO_DEVICE, "device %d out of range", dev);
   cudaError_t attr_err = cudaSuccess;
   std::call_once(g_sweep_attr[dev], [&] {
-    const void* fns[2] = {reinterpret_cast<const void*>(psweep_kernel<true>),
-                          reinterpret_cast<const void*>(psweep_kernel<false>)};
-    for (int i = 0; i < 2 && attr_err == cudaSuccess; ++i)
+    const void* fns[3] = {reinterpret_cast<const void*>(psweep_kernel<true, false>),
+                          reinterpret_cast<const void*>(psweep_kernel<false, false>),
+                          reinterpret_cast<const void*>(psweep_kernel<false, true>)};
+    for (int i = 0; i < 3 && attr_err == cudaSuccess; ++i)
       attr_err = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kSweepSmem));
+                                      static_cast<int>(kSweepSmem + (i == 2 ? kAsideSmem : 0)));
   });
   BBK_CUDA_TRY(attr_err);
   const int sms = device_sm_count();
   // every sweep launch waits for its own flag value
   int mark = 0;
   auto sweeps = [&](bool forward) -> int {
-    const void* fn = forward ? reinterpret_cast<const void*>(psweep_kernel<true>)
-                             : reinterpret_cast<const void*>(psweep_kernel<false>);
+    const bool aside = !forward && nrhs > kPlainRhs;
+    const void* fn = forward ? reinterpret_cast<const void*>(psweep_kernel<true, false>)
+                     : aside ? reinterpret_cast<const void*>(psweep_kernel<false, true>)
+                             : reinterpret_cast<const void*>(psweep_kernel<false, false>);
     constexpr int chunk = kMaxGroups * kMaxRhsChunk;
     for (int c0 = 0; c0 < nrhs; c0 += chunk) {
       SweepArgs a = A;
@@ -730,7 +764,7 @@ int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const 
       a.group_ctas = std::max(1, std::min(nblk, sms / groups));
       void* kargs[] = {&a};
       BBK_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(groups * a.group_ctas), dim3(kSolveThreads), kargs,
-                                               kSweepSmem, s));
+                                               kSweepSmem + (aside ? kAsideSmem : 0), s));
       count_launch();
     }
     return BBK_OK;

@@ -182,7 +182,8 @@ int bbk_factor_host(int n, int block_size, double* a, long long lda,
  * (the reference zeroes that column of L); a singular 2x2 pivot divides by
  * zero.  The triangular sweeps are latency-bound (one dependent step per 64
  * rows): right-hand sides go through them in groups of 8, up to 16 groups
- * side by side in a launch. */
+ * side by side in a launch.  A solution's bits do not depend on the others
+ * solved with it, except that calls with more than 32 add in another order. */
 size_t bbk_solve_workspace_size(int n, int nrhs);
 int bbk_solve_device(int n, const double* factors, long long ldf,
                      const int* perm, const int* pivot_types, int nrhs,
