@@ -1991,7 +1991,8 @@ int launch_panel(const FactorPlan& plan, int panel, cudaStream_t s) {
   const int smax = ((fixed ? plan.n : m) + plan.grid - 1) / plan.grid;
   P.coef_cap = static_cast<int>(align_up(static_cast<size_t>(plan.b) + 4, 2));
   P.smem_cols = smax;
-  P.part_pitch = fixed ? kNarrowSlots : std::min(smax, kWideSlots);
+  // (the ordered sums are not split among the warps: all of the memory is for rows)
+  P.part_pitch = ordered ? 0 : fixed ? kNarrowSlots : std::min(smax, kWideSlots);
   const size_t base = (2 * static_cast<size_t>(P.coef_cap) + 2 * static_cast<size_t>(smax) +
                        2 * static_cast<size_t>(kWarps) * P.part_pitch) * sizeof(double) +
                       (static_cast<size_t>(P.win_pad) + smax) * sizeof(int);
