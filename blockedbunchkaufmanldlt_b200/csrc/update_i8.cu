@@ -888,9 +888,11 @@ int launch_update_i8(const FactorPlan& plan, int panel, long long order, const i
   const int sms = device_sm_count();
   const long long tm = order / kTile + 2;
   const int grid = static_cast<int>(std::min<long long>(tm * (tm + 1) / 2, sms));
-  if (tm * (tm + 1) / 2 > static_cast<long long>(kMaxTiles) * grid) return BBK_OK;
-  if (plan.kpad > kMaxK || digits + mags > us_room || hs_need > 12 * plan.hstride ||
-      reinterpret_cast<uintptr_t>(hs) % 16 || reinterpret_cast<uintptr_t>(us) % 16)
+  // (what depends on the panel is above: once a factorization's panels come
+  // here, which starts with the first, they all do until `order` is too small)
+  if (tiles > static_cast<size_t>(kMaxTiles) * sms || plan.kpad > kMaxK || digits + mags > us_room ||
+      hs_need > 12 * plan.hstride || reinterpret_cast<uintptr_t>(hs) % 16 ||
+      reinterpret_cast<uintptr_t>(us) % 16)
     return BBK_OK;
   SliceArgs S{};
   S.st = plan.state;
