@@ -291,7 +291,7 @@ def digit_update_flops(n: int, blk: int, panel_end) -> float:
     f, k0 = 0.0, 0
     for e in panel_end:
         kb, m = e - k0, n - e
-        if m >= 1024 and m * blk >= 512 * 1024:
+        if m >= 1024 and m * blk >= 512 * 1024 and blk >= 64:
             f += 2.0 * kb * m * (m + 1) / 2.0
         k0 = e
     return f

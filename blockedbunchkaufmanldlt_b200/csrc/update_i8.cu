@@ -865,13 +865,16 @@ int launch_update_i8(const FactorPlan& plan, int panel, long long order, const i
                      const unsigned char** marks, cudaStream_t s) {
   *gate = nullptr;
   *marks = nullptr;
-  // Sorting out digits and scales costs about 30 us per panel whatever the
+  // Sorting out digits, scales and the bound costs about 40 us per panel whatever the
   // width, and a tile's epilogue the same for any k, so the line lies at a
   // product of order and width (n = 8000, ms per factorization with the
-  // digit update down to order 1024 / 2048 / 4096 / 6144 / never: block 256:
-  // 3.74 / 3.71 / 3.95 / 4.93 / 6.67; block 128: 6.12 / 6.02 / 6.06 / 6.61 /
-  // 7.72; block 64: 10.7 / 10.5 / 10.1 / 9.87 / 9.76).
-  if (order * plan.b < 512 * 1024 || order < 1024) return BBK_OK;
+  // digit update, without the bound, down to order 1024 / 2048 / 4096 / 6144 / never:
+  // block 256: 3.74 / 3.71 / 3.95 / 4.93 / 6.67; block 128: 6.12 / 6.02 / 6.06 /
+  // 6.61 / 7.72; block 64: 10.7 / 10.5 / 10.1 / 9.87 / 9.76), and at a width, since
+  // the FP64 kernel of a narrow panel waits for C as well (ms per factorization with
+  // digits / without: n = 24000, block 48: 407 / 377, 64: 340 / 346, 80: 302 / 330, 96:
+  // 276 / 320; n = 12000: 93.7 / 92.4, 86.6 / 86.2, 81.5 / 83.3, 77.7 / 81.6).
+  if (order * plan.b < 512 * 1024 || order < 1024 || plan.b < 64) return BBK_OK;
   const long long npad = plan.ldw;
   const size_t mags = static_cast<size_t>(npad) * plan.kpad;
   const size_t digits = kDigits * mags;
