@@ -16,9 +16,10 @@
 // The critical path per block is one flag, one fold and three 32 x 32 products.
 // Right-hand sides go in groups of eight, up to sixteen groups side by side on
 // CTAs of their own.
-// Measured: n = 10000, 1 right-hand side: 1.74 -> 1.38 ms (4.4 us per block,
-// 4.2 without the substitution's code behind the products); n = 5000, 64: 11.4 ->
-// 1.58 ms.  A block that is substituted through takes 2.7 us more.
+// Measured: n = 10000, 1 right-hand side: 1.72 -> 1.32 ms (4.2 us per block);
+// n = 5000, 64: 11.4 -> 1.58 ms.  A block that is substituted through takes 2.7
+// us more.  Orders of one block gain nothing: a sweep of n = 64 takes 11 us, 8
+// before.
 #include <algorithm>
 #include <mutex>
 
@@ -328,22 +329,32 @@ __device__ __forceinline__ void solve_triangle(const double* tri, const double* 
 template <bool kForward>
 __device__ __forceinline__ void substitute(const double* tri, int bsz, const int* pt, double x0, double x1, double* y) {
   const int i0 = threadIdx.x & 31, i1 = i0 + 32;
-  const unsigned lo = __ballot_sync(0xffffffffu, i0 < bsz && pt[i0] == 2);
-  const unsigned hi = __ballot_sync(0xffffffffu, i1 < bsz && pt[i1] == 2);
-  const unsigned long long open = static_cast<unsigned long long>(hi) << 32 | lo;  // bit k: a 2x2 starts at row k
+  const bool in0 = i0 < bsz, in1 = i1 < bsz;
+  const unsigned lo = __ballot_sync(0xffffffffu, in0 && pt[i0] == 2);
+  const unsigned hi = __ballot_sync(0xffffffffu, in1 && pt[i1] == 2);
+  const unsigned long long opens = static_cast<unsigned long long>(hi) << 32 | lo;  // bit k: a 2x2 starts at row k
+  if (!in0) x0 = 0.0;
+  if (!in1) x1 = 0.0;
   if (kForward) {
-    for (int k = 0; k < bsz; ++k) {
+    // row i takes the columns k < i, less the one that its 2x2 pivot couples
+    const int end0 = !in0 || i0 == 0 ? 0 : i0 - static_cast<int>(opens >> (i0 - 1) & 1);
+    const int end1 = !in1 ? 0 : i1 - static_cast<int>(opens >> (i1 - 1) & 1);
+#pragma unroll 4
+    for (int k = 0; k < kSB; ++k) {
+      const double e0 = tri[k * kTriPitch + i0], e1 = tri[k * kTriPitch + i1];
       const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
-      const int first = k + 1 + static_cast<int>(open >> k & 1);  // first row with a term of column k
-      if (i0 >= first) x0 = __fma_rn(-tri[k * kTriPitch + i0], xk, x0);
-      if (i1 >= first) x1 = __fma_rn(-tri[k * kTriPitch + i1], xk, x1);
+      if (k < end0) x0 = __fma_rn(-e0, xk, x0);
+      if (k < end1) x1 = __fma_rn(-e1, xk, x1);
     }
   } else {
-    for (int k = bsz - 1; k >= 0; --k) {
+    const int end0 = !in0 ? kSB : i0 + static_cast<int>(opens >> i0 & 1);
+    const int end1 = !in1 ? kSB : i1 + static_cast<int>(opens >> i1 & 1);
+#pragma unroll 4
+    for (int k = kSB - 1; k >= 0; --k) {
+      const double e0 = tri[i0 * kTriPitch + k], e1 = tri[i1 * kTriPitch + k];
       const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
-      const int last = k - 1 - static_cast<int>(k > 0 ? open >> (k - 1) & 1 : 0);
-      if (i0 <= last) x0 = __fma_rn(-tri[i0 * kTriPitch + k], xk, x0);
-      if (i1 <= last) x1 = __fma_rn(-tri[i1 * kTriPitch + k], xk, x1);
+      if (k > end0) x0 = __fma_rn(-e0, xk, x0);
+      if (k > end1) x1 = __fma_rn(-e1, xk, x1);
     }
   }
   if (i0 < bsz) y[i0] = x0;
@@ -393,8 +404,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
     // the triangle's inverse, while earlier blocks are still being solved
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (t == 0) s_grown = 0;
-    invert_unit_triangle<kForward>(tri, inv, red, &s_grown);
+    // (but for the first block's, which is waited for)
+    const bool opens = b == (kForward ? 0 : nblk - 1);
+    if (t == 0) s_grown = opens;
+    if (!opens) invert_unit_triangle<kForward>(tri, inv, red, &s_grown);
     // this block's right-hand sides, for the threads that finish them
     double yin[2];
 #pragma unroll
@@ -592,7 +605,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
     // result; then once more by substitution, as where the inverse has grown.
     // (The products run either way, the flag waits in shared memory and the
     // substitution is inline: with a branch around the products, a register for
-    // the flag or a call, n = 10000 took 1.40 to 1.47 ms.)
+    // the flag or a call, n = 10000 took 1.37 to 1.47 ms.)
     const int cc0 = t >> 5;  // this thread's right-hand side
     double* yc = A.y + static_cast<long long>(cc0) * n + b0;
     const double r0 = cc0 < nc ? ys[cc0 * kSB + lane] : 0.0, r1 = cc0 < nc ? ys[cc0 * kSB + 32 + lane] : 0.0;
