@@ -336,8 +336,9 @@ int bbk_update_trailing_block(int rows, int cols, int inner_dim,
  * its perm / pivot_types at perm + items[k].piv / pivot_types +
  * items[k].piv.  Block sizes are chosen per size bucket (n <= 32, 64, 128,
  * 256, 512, 1024); the library clamps each to what shared memory holds, and
- * BBK_UPDATE_FP64 may run a matrix in panels narrower than that, so that two
- * matrices share an SM (the same pivots; other roundings).
+ * where a block is clamped just so (orders 245, 246 and 629 to 638)
+ * BBK_UPDATE_FP64 runs it in panels one narrower, so that two matrices
+ * share an SM (the same pivots; other roundings).
  * ------------------------------------------------------------------------- */
 #define BBK_BATCH_MAX_N 1024
 #define BBK_BATCH_BUCKETS 6

@@ -1,6 +1,7 @@
 """GPU: batches with two CTAs per SM.  In the FP64 mode items whose W and U
-take more than half of an SM's shared memory are factored without keeping U,
-in a panel that may be narrower than planned: same pivots as the oracle's,
+take more than half of an SM's shared memory are factored without keeping U
+(with wide blocks, test_batched_wide_blocks_gpu.py, in a panel that may be
+narrower than planned): same pivots as the oracle's,
 backward error below 20 n eps.  A workspace of the size that one CTA per SM
 needs is still accepted."""
 import ctypes
@@ -36,7 +37,7 @@ def _check(port, plan, mats, rhs, x, perm, pt):
 
 @pytest.mark.parametrize("sizes,blocks", [
     ([195, 196, 197, 255, 256], None),                  # around half the shared memory, one slot per thread
-    ([257, 300, 383, 500, 511, 512], None),             # two; the block cut at the largest
+    ([257, 300, 383, 500, 511, 512], None),             # two
     ([513, 700, 1023, 1024, 16, 33], None),             # four
     ([256, 128, 96, 64, 65, 1], [64] * 6),              # wide blocks
     ([512, 256, 31], [32, 64, 48, 48, 24, 12]),         # the tuned table

@@ -4,12 +4,17 @@ the pivots are and the residual is within the reference's 1e-10; at the
 orders where the cluster grows (64 columns per CTA), where the first panels
 run on the grid and the last ones on a cluster, and with panels wider than a
 cluster's shared memory takes."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 from common import kkt_matrix, reconstruct, relative_error, uniform_symmetric
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 CASES = [(1, 1), (2, 1), (3, 2), (64, 16), (65, 16), (66, 64), (129, 32), (257, 31), (513, 48), (1025, 64),
          (1300, 255),  # the first panel's rows do not fit a cluster
@@ -80,15 +85,12 @@ def test_an_expired_wait_in_a_cluster_is_reported_and_the_context_survives(cuda,
 
 @pytest.mark.parametrize("slots", [97, 129, 288])
 def test_many_slots_per_cta_split_the_rows(cuda, bbk, slots):
-    # the grid panel's kernel for 97 to 288 slots per CTA, its rows split
-    # between shared and global memory (block 256 beyond 90 slots or so): the
-    # decisions' quantities agree with the ordered mode's to rounding, and the
-    # pivots where no decision is a near-tie
+    # the grid panel's kernel for 97 to 288 slots per CTA at full width, its rows
+    # split between shared and global memory (block 256 beyond 90 slots or so):
+    # a permutation and the solution's backward error
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     n = slots * sms
-    if n > 30000:
-        n = 30000 - 30000 % sms  # the check is the residual's; memory bounds the order
     g = torch.Generator(device=cuda)
     g.manual_seed(slots)
     a = torch.empty(n, n, dtype=torch.float64, device=cuda).uniform_(-1.0, 1.0, generator=g)
@@ -102,3 +104,35 @@ def test_many_slots_per_cta_split_the_rows(cuda, bbk, slots):
     r = (b.T - a @ x.T).abs().amax(0)
     berr = r / (a.abs().sum(1).amax() * x.T.abs().amax(0) + b.T.abs().amax(0))
     assert float(berr.max()) < 1e-13
+
+
+SLOTS = """
+import sys
+import numpy as np
+import torch
+import blockedbunchkaufmanldlt_b200 as bbk
+slots, b = int(sys.argv[1]), int(sys.argv[2])
+n = slots * (-(-3700 // slots))  # beyond a cluster's columns at first
+rng = np.random.default_rng(slots)
+a = np.triu(rng.uniform(-1.0, 1.0, (n, n)))
+a = torch.from_numpy(a + np.triu(a, 1).T).cuda()
+out = []
+for mode in ("fp64", "fp64_ordered"):
+    f = a.clone()
+    out.append((f,) + bbk.factor_device(f, b, mode=mode))
+for k in (1, 2, 3):
+    assert torch.equal(out[0][k], out[1][k]), ("perm", "pivot types", "panel ends")[k - 1]
+u, w = (torch.triu(o[0]) for o in out)
+assert float((u - w).norm() / w.norm()) < 1e-10
+"""
+
+
+@pytest.mark.parametrize("slots,b", [(96, 64), (97, 64), (224, 128), (257, 64), (288, 64), (288, 300), (289, 64)])
+def test_slots_per_cta_pivot_as_the_ordered_mode(cuda, bbk, slots, b):
+    # fewer CTAs, so that each has as many slots at an order where the pivots
+    # can be compared: 96 and 97, 257 and 288 (nine chunks), 289 (one thread per
+    # slot again), rows in shared and (block 300) in global memory
+    env = {**os.environ, "BBK_PANEL_COLS": str(slots), "PYTHONPATH": ROOT}
+    run = subprocess.run([sys.executable, "-c", SLOTS, str(slots), str(b)], env=env, capture_output=True, text=True,
+                         timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]

@@ -37,7 +37,8 @@ def _scaled(a, spread, seed):
     (2432, 255, 0, "random"),   # odd width: k padded inside a chunk
     (2559, 257, 1, "random"),   # odd order, even leading dimension, k in nine chunks
     (1664, 512, 2, "kkt"),
-    (1800, 900, 0, "random"),   # a wide panel: k = 900, two of them
+    (2100, 900, 0, "random"),   # a wide panel: k = 900
+    (2200, 1000, 0, "random"),  # nearly the widest, k = 1000
     (4400, 130, 0, "kkt"),
     (2306, 256, 0, "scaled3"),  # rows and columns spread over 10^+-3, 10^+-30
     (2306, 256, 0, "scaled30"),
@@ -47,11 +48,17 @@ def test_digit_update_has_the_oracles_pivots_and_residual(cuda, bbk, port, n, b,
     if kind.startswith("scaled"):
         a = _scaled(a, float(kind[6:]), 3)
     want = port.factor(a, b)
+    launches = [bbk.kernel_launch_count()]
     f, perm, pt, ends = _factor(bbk, cuda, a, b, pad=pad)
+    launches.append(bbk.kernel_launch_count())
     assert np.array_equal(pt.cpu().numpy(), want.pivot_types)
     assert np.array_equal(perm.cpu().numpy(), want.perm)
     assert np.array_equal(ends.cpu().numpy(), want.panel_end)
     fo, po, to, _ = _factor(bbk, cuda, a, b, mode="fp64_ordered", pad=pad)
+    launches.append(bbk.kernel_launch_count())
+    # the digit kernels ran: four launches more for each panel above the line
+    above = [m for m in range(n - b + 1, b, -b) if m >= 1024 and m * b >= 1 << 19]
+    assert above and launches[1] - launches[0] == launches[2] - launches[1] + 4 * len(above)
     assert _residual(bbk, a, f, perm, pt) <= 2.0 * _residual(bbk, a, fo, po, to)
 
 

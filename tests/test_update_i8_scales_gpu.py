@@ -29,8 +29,9 @@ def _residual_by_entry(a, f, perm, pt, rows):
 
     wide = [v.astype(np.longdouble) for v in (l, lt, d, off)]
     r = np.abs(a[np.ix_(perm[rows], perm)] - product(*wide))
-    # (in double: the bound needs no more)
-    return float((r / product(*(np.abs(v) for v in (l, lt, d, off)))).max())
+    size = product(*(np.abs(v) for v in (l, lt, d, off)))  # (in double: it needs no more)
+    assert not r[size == 0.0].any()
+    return float((r[size > 0.0] / size[size > 0.0]).max())
 
 
 def _factor(bbk, cuda, a, b, mode):
@@ -58,13 +59,27 @@ def _few_rows(n, scale):
     return a
 
 
+def _flat(n, scale):
+    # pivots that do not couple, then rows of entries close to the largest that
+    # the leading digit holds, all of one sign: the digits' sums are at their largest
+    rng = np.random.default_rng(23)
+    a = uniform_symmetric(n, 23)
+    h = 1000
+    a[:h, :h] = np.diag(np.full(h, 10.0))
+    a[:h, h:] = rng.uniform(0.9925, 0.9955, (h, n - h))
+    a[h:, :h] = a[:h, h:].T
+    a[h:, h:] += a[h:, :h] @ a[:h, h:] / 10.0  # (what the update takes off again)
+    return a
+
+
 @pytest.mark.parametrize("kind,scale,n,b", [
+    ("flat", 1.0, 2100, 1000), ("flat", 1.0, 2200, 500),
     ("two", 1.0, 2304, 256), ("two", 1e2, 2304, 256), ("two", 1e4, 2304, 256), ("two", 1e6, 2304, 256),
     ("two", 1e10, 2304, 256), ("two", 1e5, 2450, 305), ("two", 1e6, 3000, 600), ("two", 1e6, 2200, 1000),
     ("two", 1e6, 8300, 64), ("few", 1e4, 2304, 256), ("few", 1e8, 2304, 256),
 ])
 def test_every_entry_is_as_accurate_as_in_the_references_order(cuda, bbk, kind, scale, n, b):
-    a = (_two_sets if kind == "two" else _few_rows)(n, scale)
+    a = {"two": _two_sets, "few": _few_rows, "flat": _flat}[kind](n, scale)
     got = []
     for mode in ("fp64", "fp64_ordered"):
         f, perm, pt = (t.cpu().numpy() for t in _factor(bbk, cuda, a, b, mode))
