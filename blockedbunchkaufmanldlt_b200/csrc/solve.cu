@@ -17,7 +17,7 @@
 // Right-hand sides go in groups of eight, up to sixteen groups side by side on
 // CTAs of their own.
 // Measured: n = 10000, 1 right-hand side: 1.72 -> 1.32 ms (4.2 us per block);
-// n = 5000, 64: 11.4 -> 1.58 ms.  A block that is substituted through takes 2.7
+// n = 5000, 64: 11.4 -> 1.51 ms.  A block that is substituted through takes 2.7
 // us more.  Orders of one block gain nothing: a sweep of n = 64 takes 11 us, 8
 // before.
 #include <algorithm>
@@ -38,14 +38,14 @@ constexpr int kMaxRhsChunk = 8;   // right-hand sides of a group
 // 49 / 44 / 43; a sweep that reads the factor once for all of them: 11.4 and
 // 162).
 constexpr int kMaxGroups = 16;
-// Beyond this many right-hand sides the backward sweep sets the sums of every
-// kWindow blocks aside.  A lane's one running sum over all columns has an
-// error that grows with n: mean backward error of 64 right-hand sides, n = 2000,
-// 5000, 10000: 7.1e-16, 1.4e-15, 2.4e-15, with the sums set aside 6.8e-16, 1.0e-15,
-// 1.3e-15 (the sweep that read the factor once for all of them, and subtracted block
-// by block: 6.8e-16, 1.0e-15, 1.5e-15).  It takes 9 % longer (n = 5000, 64: 1.45 ->
-// 1.57 ms), with one right-hand side 15 %, so up to kPlainRhs, where the sums never were
-// split, they are not.
+// Beyond this many right-hand sides the backward sweep adds the sums of every
+// kWindow blocks over the lanes and sets them aside.  A lane's one running sum over
+// all columns has an error that grows with n: mean backward error of 64 right-hand
+// sides, n = 2000, 5000, 10000: 7.1e-16, 1.4e-15, 2.4e-15, with the sums set aside
+// 7.0e-16, 1.0e-15, 1.3e-15 (the sweep that read the factor once for all of them, and
+// subtracted block by block: 6.8e-16, 1.0e-15, 1.5e-15).  It takes 4 % longer (n =
+// 5000, 64: 1.45 -> 1.51 ms; with the lanes' sums kept apart in shared memory
+// 1.58).  Up to kPlainRhs the sums never were split, and are not.
 constexpr int kPlainRhs = 32;
 constexpr int kWindow = 16;
 constexpr int kAhead = 4;         // factor blocks prefetched into L2 ahead of the fold
@@ -125,8 +125,6 @@ constexpr int kTriPitch = kSB + 1;
 constexpr int kInvTmp = 2 * 16 * 17;  // scratch of invert_unit_triangle, doubles
 static_assert(kInvTmp <= 4 * kMaxRhsChunk * kSB, "it fits the partial sums' space");
 constexpr size_t kSweepSmem = (2 * kSB * kTriPitch + 4 * kMaxRhsChunk * kSB + kMaxRhsChunk * kSB) * sizeof(double);
-constexpr size_t kAsideSmem = 8 * kMaxRhsChunk * kSolveThreads * sizeof(double);  // the sums set aside
-static_assert(kSweepSmem + kAsideSmem <= 227 * 1024, "they fit the shared memory of one CTA");
 
 // One sweep for up to kMaxGroups groups of kMaxRhsChunk right-hand sides, each
 // with CTAs and flags of its own.  CTA c of a group owns blocks c, c+G, ... in
@@ -368,7 +366,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
   double* inv = tri + kSB * kTriPitch;          // its inverse
   double* red = inv + kSB * kTriPitch;          // [4][kMaxRhsChunk][kSB] partial sums
   double* ys = red + 4 * kMaxRhsChunk * kSB;    // [kMaxRhsChunk][kSB]: the block being solved
-  double* aside = ys + kMaxRhsChunk * kSB;      // [8][kMaxRhsChunk][kSolveThreads] (kAside)
   __shared__ int s_fail, s_grown;
   const int n = A.n;
   const long long ldf = A.ldf;
@@ -495,6 +492,31 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
       for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int cc = 0; cc < kMaxRhsChunk; ++cc) acc[j][cc] = 0.0;
+      // add the 64 sums of (j, cc) over the lanes by recursive halving: at
+      // offset o each lane keeps one half of its values and adds the
+      // partner's copy of that half; after five levels lane l holds the
+      // totals of entries 2l and 2l + 1 (62 shuffles, depth 5)
+      static_assert(8 * kMaxRhsChunk == 64, "the halving below assumes 64 sums per lane");
+      auto add_lanes = [&](double& s0, double& s1) {
+        double v[64];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int cc = 0; cc < kMaxRhsChunk; ++cc) v[j * kMaxRhsChunk + cc] = acc[j][cc];
+#pragma unroll
+        for (int o = 16, m = 64; o > 0; o >>= 1, m >>= 1) {
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int e = 0; e < m / 2; ++e) {
+            const double send = up ? v[e] : v[e + m / 2];
+            const double keep = up ? v[e + m / 2] : v[e];
+            v[e] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        }
+        s0 = v[0];
+        s1 = v[1];
+      };
+      double aside0 = 0.0, aside1 = 0.0;  // the totals of the windows before
       auto load_f = [&](int k, double (&l)[16]) {
         const int k0 = k * kSB;
         const bool edge = k == b + 1 && b0 + kSB - 1 < n && A.pt[b0 + kSB - 1] == 2;
@@ -538,43 +560,21 @@ __global__ void __launch_bounds__(kSolveThreads, 1) psweep_kernel(SweepArgs A) {
 #pragma unroll
         for (int u = 0; u < 16; ++u) fc[u] = fn[u];
         if (kAside && (k_first - k) % kWindow == kWindow - 1 && k > k_end) {
+          double s0, s1;
+          add_lanes(s0, s1);
+          aside0 += s0;
+          aside1 += s1;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
 #pragma unroll
-            for (int cc = 0; cc < kMaxRhsChunk; ++cc)
-              if (cc < nc) {
-                double* sum = aside + (j * kMaxRhsChunk + cc) * kSolveThreads + t;
-                *sum = k_first - k < kWindow ? acc[j][cc] : *sum + acc[j][cc];
-                acc[j][cc] = 0.0;
-              }
+            for (int cc = 0; cc < kMaxRhsChunk; ++cc) acc[j][cc] = 0.0;
         }
       }
-      if (kAside && k_first - k_end >= kWindow) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int cc = 0; cc < kMaxRhsChunk; ++cc)
-            if (cc < nc) acc[j][cc] += aside[(j * kMaxRhsChunk + cc) * kSolveThreads + t];
-      }
-      // add the 64 sums of (j, cc) over the lanes by recursive halving: at
-      // offset o each lane keeps one half of its values and adds the
-      // partner's copy of that half; after five levels lane l holds the
-      // totals of entries 2l and 2l + 1 (62 shuffles, depth 5)
-      static_assert(8 * kMaxRhsChunk == 64, "the halving below assumes 64 sums per lane");
-      double v[64];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int cc = 0; cc < kMaxRhsChunk; ++cc) v[j * kMaxRhsChunk + cc] = acc[j][cc];
-#pragma unroll
-      for (int o = 16, m = 64; o > 0; o >>= 1, m >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int e = 0; e < m / 2; ++e) {
-          const double send = up ? v[e] : v[e + m / 2];
-          const double keep = up ? v[e + m / 2] : v[e];
-          v[e] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
+      double v[2];
+      add_lanes(v[0], v[1]);
+      if (kAside) {
+        v[0] += aside0;
+        v[1] += aside1;
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -756,7 +756,7 @@ int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const 
                           reinterpret_cast<const void*>(psweep_kernel<false, true>)};
     for (int i = 0; i < 3 && attr_err == cudaSuccess; ++i)
       attr_err = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kSweepSmem + (i == 2 ? kAsideSmem : 0)));
+                                      static_cast<int>(kSweepSmem));
   });
   BBK_CUDA_TRY(attr_err);
   const int sms = device_sm_count();
@@ -777,7 +777,7 @@ int solve_enqueue(int n, const double* f, long long ldf, const int* perm, const 
       a.group_ctas = std::max(1, std::min(nblk, sms / groups));
       void* kargs[] = {&a};
       BBK_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(groups * a.group_ctas), dim3(kSolveThreads), kargs,
-                                               kSweepSmem + (aside ? kAsideSmem : 0), s));
+                                               kSweepSmem, s));
       count_launch();
     }
     return BBK_OK;
