@@ -421,13 +421,14 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Bounded wait for phase `phase` of a barrier in this CTA's shared memory.
+// Bounded wait for phase `phase` of a barrier in this CTA's shared memory (at
+// cluster scope: what it guards was stored by other CTAs).
 __device__ __forceinline__ bool cluster_wait(const PanelArgs& P, uint32_t bar, uint32_t phase) {
   unsigned long long t0 = 0;
   for (unsigned iter = 1;; ++iter) {
     uint32_t done;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(done)
         : "r"(bar), "r"(phase)
