@@ -29,7 +29,7 @@
 // panel with more than half of its tiles left so goes there whole).  Against
 // |L| |D| |L^T|, in units of 2^-53, n = 2304, block 256, two index sets at scales s
 // and 1 coupled by entries of size 1: digits alone 2.6, 45 and 4485 at s = 10^3,
-// 10^4 and 10^6; with the bound 1.3, 2.4 and 2.5, the same as the FP64 tensor cores alone.
+// 10^4 and 10^6; with the bound 1.3, 2.4 and 2.5, as the FP64 tensor cores alone.
 // The random, KKT and spectral matrices timed here need 5 to 15 of the 16, a
 // few tiles of a KKT matrix's first panel more.
 //
@@ -41,9 +41,9 @@
 // FP64 tensor-core kernel, which is launched behind this one and returns
 // unless the flag is set.
 //
-// Measured (B200): update at n = 40000, block 256: 758 -> 321 ms per
-// factorization (12 of them the bound); n = 16000, block 256: 48.9 -> 23.4 ms;
-// n = 10000, block 128: 13.9 -> 11.1 ms.
+// Measured (B200): update at n = 40000, block 256: 758 -> 317 ms per
+// factorization (13 of them the bound); n = 16000, block 256: 48.9 -> 22.4 ms;
+// n = 10000, block 128: 13.9 -> 10.9 ms.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
